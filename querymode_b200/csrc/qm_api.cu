@@ -1019,6 +1019,7 @@ struct Exec {
   int dedupe = 1;
   int strategy = 0;
   int priv = 0;  // direct block-local table copied per warp (no atomics)
+  int local_rep = 0;  // log2 of the copies of each direct block-local slot
 };
 
 int64_t special_slots(int mode) { return mode == QK_HASH ? 2 : (mode == QK_DIRECT ? 1 : 0); }
@@ -1039,6 +1040,17 @@ constexpr size_t DIRECT_LOCAL_BUDGET = 180 * 1024;
 // Bytes of all per-warp copies of a small direct table.
 constexpr size_t PRIV_BUDGET = 64 * 1024;
 constexpr int64_t PRIV_MIN_ROWS = (int64_t)8 << 20;
+// Bytes of all copies of a small direct block-local table.  A shared-memory
+// atomic that returns its old value serialises on equal addresses (31 cycles a
+// warp on one slot, 5 on 16), so few slots are copied, up to a copy per lane.
+constexpr int64_t REP_BUDGET = 24 * 1024;
+
+// log2 of the copies of `slots` slots of `per_slot` bytes.
+int local_copies(int64_t slots, int64_t per_slot) {
+  int r = 0;
+  while (r < 5 && (slots << (r + 1)) * per_slot <= REP_BUDGET) r++;
+  return r;
+}
 
 void choose_layout(const Plan &pl, int64_t est_groups, Exec &ex, const qm_tuning &tu) {
   const int words = pl.agg.n_words;
@@ -1046,21 +1058,21 @@ void choose_layout(const Plan &pl, int64_t est_groups, Exec &ex, const qm_tuning
   ex.total_slots = ex.n_slots + special_slots(pl.key.mode);
   const int64_t per_slot = (int64_t)words * 8;
   ex.priv = 0;
+  ex.local_rep = 0;
   if (pl.key.mode == QK_NONE) {
-    ex.local_slots = 1;
+    ex.dedupe = tu.dedupe > 0;
+    ex.priv = ex.dedupe;
+    if (!ex.dedupe) ex.local_rep = local_copies(1, per_slot);
+    ex.local_slots = 1 << ex.local_rep;
     ex.local_hash = 0;
-    ex.dedupe = 1;
-    ex.priv = 1;
     ex.strategy = 0;
     return;
   }
   if (pl.key.mode == QK_DIRECT && tu.local_slots >= 0 && (ex.n_slots + 1) * per_slot <= (int64_t)DIRECT_LOCAL_BUDGET) {
-    ex.local_slots = (int)(ex.n_slots + 1);
     ex.local_hash = 0;
-    // warp deduplication is off by default for dense keys: the scan's own
-    // equal-slot merge costs fewer instructions (measured 2.5x faster at 11
-    // groups, 1.5x at 16)
     ex.dedupe = tu.dedupe >= 0 ? tu.dedupe : 0;
+    if (!ex.dedupe) ex.local_rep = local_copies(ex.n_slots + 1, per_slot);
+    ex.local_slots = (int)(ex.n_slots + 1) << ex.local_rep;
     // deduplicated rows have distinct slots within a warp, so a small table
     // copied per warp is then updated without atomics
     ex.priv = ex.dedupe && (ex.n_slots + 1) * per_slot * (QM_SCAN_THREADS / 32) <= (int64_t)PRIV_BUDGET;
@@ -1282,6 +1294,15 @@ int plan_split_sums(qm_ctx *ctx, Plan &pl, int64_t n_rows, bool deterministic) {
     }
     if (e + k > 1000 || e + k < -960) continue;  // keep TwoSum at the ends of the range
     vc.split = 1.5 * std::ldexp(1.0, e + k);
+    // the block-local integers (local_fsum): a multiple of 2^(p - 52) below
+    // 2^(62 - b), the rest a multiple of 2^(q - 52) below 2^(62 - b)
+    const int b = std::max(k, 12), p = e + b - 10, q = p + b - 63;
+    vc.lim = std::ldexp(1.0, e);
+    vc.sa = std::ldexp(1.5, p);
+    vc.sb = std::ldexp(1.5, q);
+    vc.ga = std::ldexp(1.0, p - 52);
+    vc.gb = std::ldexp(1.0, q - 52);
+    vc.lsh = 10 + k - b;
   }
   return QM_OK;
 }
@@ -1444,6 +1465,7 @@ void fill_args(const GroupTable &gt, qm_scan_args &a, qm_status *st) {
   a.local_hash = gt.ex.local_hash;
   a.dedupe = gt.ex.dedupe;
   a.priv = gt.ex.priv;
+  a.local_rep = gt.ex.local_rep;
   a.zones = gt.zones;
   a.n_zone_tiles = gt.n_zone_tiles;
   a.max_probe = 1 << 12;
@@ -3773,6 +3795,11 @@ int batch_layout(qm_batch *b) {
     const int64_t per_slot = (int64_t)gt.pl.agg.n_words * 8;
     if (ex.local_slots > 0) {
       int64_t need = (int64_t)ex.local_slots * (per_slot + (ex.local_hash ? 8 : 0));
+      while (ex.local_rep > 0 && need > (int64_t)local_budget) {  // fewer copies of each slot
+        ex.local_rep--;
+        ex.local_slots >>= 1;
+        need >>= 1;
+      }
       if (local_budget == 0) {
         ex.local_slots = 0;
       } else if (need > (int64_t)local_budget) {

@@ -58,29 +58,14 @@ __global__ void qm_batch_init(const qm_bq *bq, const int64_t *slot0, int n, int6
 // Shared memory: block-local table (keys, then words SoA), per-warp queues,
 // per-warp merge scratch — sized for the batch's largest local table.
 struct bsmem {
-  size_t words_off, queue_off, scratch_off, bytes;
+  size_t words_off, queue_off, bytes;
 };
 __host__ __device__ inline bsmem batch_smem(int local_bytes, int warps) {
   bsmem s;
   s.words_off = 0;
   s.queue_off = ((size_t)local_bytes + 15) & ~(size_t)15;
-  s.scratch_off = s.queue_off + (size_t)warps * (QM_TILE_ROWS + 32) * sizeof(uint32_t);
-  s.bytes = s.scratch_off + (size_t)warps * 64 * sizeof(uint64_t);
+  s.bytes = s.queue_off + (size_t)warps * (QM_TILE_ROWS + 32) * sizeof(uint32_t);
   return s;
-}
-
-__device__ void batch_flush(const qm_scan_args &a, uint64_t *lkeys, uint64_t *lw) {
-  const int L = a.local_slots;
-  if (L <= 0) return;
-  const qm_aggspec &A = a.agg;
-  for (int s = threadIdx.x; s < L; s += blockDim.x) {
-    if (lw[(int64_t)A.w_count * L + s] == 0) continue;
-    int64_t gs;
-    if (a.local_hash) gs = global_slot(a, lkeys[s], 0);
-    else gs = s;
-    if (gs < 0) continue;
-    merge_local(A, lw + s, L, a.table + gs * a.stride + 1);
-  }
 }
 
 // DD / NV / KK: the dedupe flag, value-column count and key kind of the
@@ -99,7 +84,6 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   const int warps = blockDim.x >> 5;
   const bsmem lay = batch_smem(local_bytes, warps);
   uint32_t *queue = reinterpret_cast<uint32_t *>(smem + lay.queue_off) + warp * (QM_TILE_ROWS + 32);
-  uint64_t *scr = reinterpret_cast<uint64_t *>(smem + lay.scratch_off) + warp * 64;
   uint64_t *lkeys = reinterpret_cast<uint64_t *>(smem);
   uint64_t *lw = lkeys;
   int cur = -1;
@@ -113,7 +97,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
     const qm_chunk ch = chunks[c];
     if (ch.q != cur) {
       if (cur >= 0) {
-        batch_flush(P, lkeys, lw);
+        merge_block(P, lkeys, lw);
         if (lane == 0 && selected) atomicAdd(&P.status->rows_selected, selected);
         selected = 0;
       }
@@ -173,19 +157,19 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
         const int64_t row = queue[qn - 32 + lane];
         __syncwarp();
         qn -= 32;
-        drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS)>(P, lkeys, lw, L, &l_used, lane, true, row, scr);
+        drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, &l_used, lane, true, row);
       }
     }
     if (qn > 0) {
       const bool active = lane < qn;
       const int64_t row = active ? (int64_t)queue[lane] : 0;
       __syncwarp();
-      drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS)>(P, lkeys, lw, L, &l_used, lane, active, row, scr);
+      drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, &l_used, lane, active, row);
     }
     __syncthreads();
   }
   if (cur >= 0) {
-    batch_flush(P, lkeys, lw);
+    merge_block(P, lkeys, lw);
     if (lane == 0 && selected) atomicAdd(&P.status->rows_selected, selected);
   }
 }

@@ -1200,12 +1200,12 @@ cudaError_t scan_attrs_once() {
   if (dev < 64 && done[dev]) return cudaSuccess;
 #define QM_SMEM_ATTR(K) \
   if (e == cudaSuccess) e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, QM_SCAN_SMEM_MAX);
-  QM_SMEM_ATTR((qm_scan_kernel<false, true, 0, QM_NV_ANY, QM_KK_ANY>));
-  QM_SMEM_ATTR((qm_scan_kernel<false, true, 1, QM_NV_ANY, QM_KK_ANY>));
-  QM_SMEM_ATTR((qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY>));
-  QM_SMEM_ATTR((qm_scan_kernel<false, false, 1, QM_NV_ANY, QM_KK_ANY>));
-  QM_SMEM_ATTR((qm_scan_kernel<true, false, 0, QM_NV_ANY, QM_KK_ANY>));
-  QM_SMEM_ATTR((qm_scan_kernel<true, false, 1, QM_NV_ANY, QM_KK_ANY>));
+  QM_SMEM_ATTR((qm_scan_kernel<false, true, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
+  QM_SMEM_ATTR((qm_scan_kernel<false, true, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
+  QM_SMEM_ATTR((qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
+  QM_SMEM_ATTR((qm_scan_kernel<false, false, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
+  QM_SMEM_ATTR((qm_scan_kernel<true, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
+  QM_SMEM_ATTR((qm_scan_kernel<true, false, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
 #undef QM_SMEM_ATTR
   if (e == cudaSuccess) e = qm_scan_nv0_attr(QM_SCAN_SMEM_MAX);
   if (e == cudaSuccess) e = qm_scan_nv1_attr(QM_SCAN_SMEM_MAX);
@@ -1225,6 +1225,21 @@ int key_kind(const qm_keyspec &K) {
   }
   return QM_KK_ANY;
 }
+
+// The most restricted set of paths (QM_FT_*) the plan's value columns need.
+int value_features(const qm_aggspec &A) {
+  int ft = QM_FT_SUM;
+  for (int c = 0; c < A.n_vcols; ++c) {
+    const qm_vcol &vc = A.vcol[c];
+    const bool isint = vc.dtype == QM_I32 || vc.dtype == QM_I64;
+    if (vc.flags & VF_FIXED) return QM_FT_FULL;
+    if (vc.nulls || (vc.flags & (VF_NN | VF_WIDE)) || (!isint && (vc.flags & VF_SUM) && vc.split == 0.0))
+      ft = QM_FT_GEN;
+    else if (isint || (vc.flags & (VF_SUM | VF_MIN | VF_MAX | VF_ZERO)) != VF_SUM)
+      ft = ft < QM_FT_MIX ? ft : QM_FT_MIX;
+  }
+  return ft;
+}
 }  // namespace
 
 cudaError_t qm_scan_configure(size_t smem_bytes, bool staged, int *blocks_per_sm) {
@@ -1233,9 +1248,9 @@ cudaError_t qm_scan_configure(size_t smem_bytes, bool staged, int *blocks_per_sm
   if (e != cudaSuccess) return e;
   if (staged)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        blocks_per_sm, qm_scan_kernel<false, true, 0, QM_NV_ANY, QM_KK_ANY>, QM_SCAN_THREADS, smem_bytes);
+        blocks_per_sm, qm_scan_kernel<false, true, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>, QM_SCAN_THREADS, smem_bytes);
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      blocks_per_sm, qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY>, QM_SCAN_THREADS, smem_bytes);
+      blocks_per_sm, qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>, QM_SCAN_THREADS, smem_bytes);
 }
 
 cudaError_t qm_launch_scan(const qm_scan_args &a, int blocks, size_t smem_bytes, cudaStream_t st) {
@@ -1243,29 +1258,29 @@ cudaError_t qm_launch_scan(const qm_scan_args &a, int blocks, size_t smem_bytes,
   cudaError_t e = scan_attrs_once();
   if (e != cudaSuccess) return e;
   const int dd = a.dedupe != 0 ? 1 : 0;
-  // fixed-point (deterministic) sums run in the run-time-plan kernels only
-  bool fixed = false;
-  for (int c = 0; c < a.agg.n_vcols; ++c) fixed = fixed || (a.agg.vcol[c].flags & VF_FIXED) != 0;
-  if (!a.sel && a.stage.n == 0 && a.agg.n_vcols <= QM_SPEC_NV_MAX && !fixed) {
-    int kk = key_kind(a.key);
-    if (kk == QM_KK_NONE && !dd) kk = QM_KK_ANY;
-    switch (a.agg.n_vcols) {
-      case 0: return qm_scan_nv0_launch(a, dd, kk, blocks, smem_bytes, st);
-      case 1: return qm_scan_nv1_launch(a, dd, kk, blocks, smem_bytes, st);
-      case 2: return qm_scan_nv2_launch(a, dd, kk, blocks, smem_bytes, st);
-      case 3: return qm_scan_nv3_launch(a, dd, kk, blocks, smem_bytes, st);
-      case 4: return qm_scan_nv4_launch(a, dd, kk, blocks, smem_bytes, st);
+  if (!a.sel && a.stage.n == 0 && a.agg.n_vcols <= QM_SPEC_NV_MAX) {
+    const int ft = value_features(a.agg);
+    if (ft != QM_FT_FULL) {  // fixed-point (deterministic) sums run in the run-time-plan kernels only
+      const int kk = dd ? QM_KK_ANY : key_kind(a.key);
+      const int lm = !dd && a.local_slots > 0 && !a.local_hash ? QM_LM_DIRECT : QM_LM_ANY;
+      switch (a.agg.n_vcols) {
+        case 0: return qm_scan_nv0_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
+        case 1: return qm_scan_nv1_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
+        case 2: return qm_scan_nv2_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
+        case 3: return qm_scan_nv3_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
+        case 4: return qm_scan_nv4_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
+      }
     }
   }
   if (a.sel) {
-    if (dd) qm_scan_kernel<true, false, 1, QM_NV_ANY, QM_KK_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
-    else qm_scan_kernel<true, false, 0, QM_NV_ANY, QM_KK_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
+    if (dd) qm_scan_kernel<true, false, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
+    else qm_scan_kernel<true, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
   } else if (a.stage.n > 0) {
-    if (dd) qm_scan_kernel<false, true, 1, QM_NV_ANY, QM_KK_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
-    else qm_scan_kernel<false, true, 0, QM_NV_ANY, QM_KK_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
+    if (dd) qm_scan_kernel<false, true, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
+    else qm_scan_kernel<false, true, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
   } else {
-    if (dd) qm_scan_kernel<false, false, 1, QM_NV_ANY, QM_KK_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
-    else qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
+    if (dd) qm_scan_kernel<false, false, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
+    else qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
   }
   return cudaGetLastError();
 }

@@ -8,9 +8,9 @@
 //   2. compaction: __ballot_sync masks + popcount prefix sums put the
 //      surviving row offsets, in ascending row order, into a per-warp list;
 //   3. aggregation: 32 survivors at a time, the lane gathers its row's key and
-//      value cells, equal keys in the warp are merged with __match_any_sync
-//      (one update per distinct key), and the leader updates the block-local
-//      shared-memory table (or the global table when the key misses it).
+//      value cells and updates the block-local shared-memory table (or the
+//      global table when the key misses it).  The block-local words are built
+//      from native 32-bit shared-memory atomics (see agg_row_local).
 // At block end the shared-memory table is merged into the global table with
 // atomics.  Float sums are compensated (TwoSum of every atomic add: the old
 // value returned by atomicAdd gives the exact rounding error, which goes to a
@@ -429,6 +429,19 @@ __device__ __forceinline__ uint32_t eval_pred(const qm_pred &P, const ROWS &row,
 // plan's n_vcols at run time).
 #define QM_NV_ANY (QM_MAX_VCOLS + 1)
 #define QM_NV_BOUND(NV) ((NV) > QM_MAX_VCOLS ? QM_MAX_VCOLS : (NV))
+// What the value columns of a plan can need (FT): 0 anything, fixed-point
+// sums included; 1 anything but those; 2 no NULLs, no 128-bit integer sums,
+// float sums split (planned from statistics); 3 as 2, and every column is a
+// float one with a SUM only.  A path a kernel leaves out costs its drain no
+// instructions: the flags are tested once per row and column otherwise.
+#define QM_FT_FULL 0
+#define QM_FT_GEN 1
+#define QM_FT_MIX 2
+#define QM_FT_SUM 3
+// Where rows go (LM): 0 as planned; 1 every row has a slot of the
+// block-local table (a dense key range, or no GROUP BY).
+#define QM_LM_ANY 0
+#define QM_LM_DIRECT 1
 
 // The payload columns of a tile (key columns, then value columns) into L2
 // ahead of the survivors' gathers.
@@ -566,7 +579,10 @@ __device__ __forceinline__ int64_t find_slot(const qm_scan_args &a, uint64_t key
 // most half full (`used` counts admissions), so a miss meets an empty slot
 // within a few probes and goes to the global table.
 __device__ __forceinline__ int local_find(uint64_t *lkeys, int L, uint64_t key, int *used) {
-  uint32_t s = (uint32_t)fmix64(key) & (uint32_t)(L - 1);
+  // a multiplicative hash of the folded key: this table only fronts the
+  // global one, so a poor spread costs misses, not correctness
+  uint32_t s = ((uint32_t)key * 0x9e3779b1u) ^ ((uint32_t)(key >> 32) * 0x85ebca6bu);
+  s = (s ^ (s >> 15)) & (uint32_t)(L - 1);
   for (int p = 0; p < QM_LOCAL_PROBE; ++p) {
     uint64_t k = reinterpret_cast<volatile uint64_t *>(lkeys)[s];
     if (k == key) return (int)s;
@@ -1017,218 +1033,209 @@ __device__ __forceinline__ void apply_row(const qm_aggspec &A, uint64_t *tp, int
   }
 }
 
-// One row's update of the slot whose word w lives at tp[w * ws]: straight
+// One row's update of the global slot whose words start at tp: straight
 // line per value column, values already gathered into vb (NULL bits in
-// vnull) so the cell loads overlap the key lookup.
-#ifndef QM_GLOBAL_READ_TEST
-#define QM_GLOBAL_READ_TEST 0
-#endif
-template <int NV = QM_NV_ANY, bool FX = true>
-__device__ __forceinline__ void agg_row(const qm_aggspec &A, uint64_t *tp, int ws, bool local,
-                                        uint64_t grow, const uint64_t (&vb)[QM_MAX_VCOLS], uint32_t vnull,
-                                        qm_status *st = nullptr) {
-  // In the global table, the FIRST word and the MIN / MAX words of the first
-  // two value columns are read up front, in one L2 round trip; the atomics
-  // then go out only where the row beats the word read.  A word only moves
-  // one way, so a stale read can cause an unneeded atomic, never skip one.
-  uint64_t g_first = 0;
-  int64_t g_mn[2] = {0, 0}, g_mx[2] = {0, 0};
-  const bool gtest = QM_GLOBAL_READ_TEST && !local;
-  if (gtest) {
-    if (A.w_first >= 0) g_first = __ldcg(reinterpret_cast<const unsigned long long *>(tp + (int64_t)A.w_first * ws));
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      if (c >= A.n_vcols) break;
-      const int f = A.vcol[c].flags;
-      if (f & VF_MIN) g_mn[c] = __ldcg(reinterpret_cast<const long long *>(tp + (int64_t)A.vcol[c].w_min * ws));
-      if (f & VF_MAX) g_mx[c] = __ldcg(reinterpret_cast<const long long *>(tp + (int64_t)A.vcol[c].w_max * ws));
-    }
-  }
-  atomicAdd(reinterpret_cast<unsigned long long *>(tp + (int64_t)A.w_count * ws), 1ULL);
-  if (A.w_first >= 0) {
-    uint64_t *p = tp + (int64_t)A.w_first * ws;
-    if (!gtest) upd_min_u64(p, grow, local);
-    else if (grow < g_first) atomicMin(reinterpret_cast<unsigned long long *>(p), (unsigned long long)grow);
-  }
-  auto gmin = [&](int c, uint64_t *p, int64_t v) {
-    if (gtest && c < 2) {
-      if (v < g_mn[c]) atomicMin(reinterpret_cast<long long *>(p), (long long)v);
-    } else {
-      upd_min_i64(p, v, local);
-    }
-  };
-  auto gmax = [&](int c, uint64_t *p, int64_t v) {
-    if (gtest && c < 2) {
-      if (v > g_mx[c]) atomicMax(reinterpret_cast<long long *>(p), (long long)v);
-    } else {
-      upd_max_i64(p, v, local);
-    }
-  };
+// vnull) so the cell loads overlap the key lookup.  The atomics return
+// nothing (fire-and-forget reductions): a read test would cost an L2 round
+// trip that the warp waits for.
+template <int NV = QM_NV_ANY, int FT = QM_FT_FULL>
+__device__ __forceinline__ void agg_row(const qm_aggspec &A, uint64_t *tp, uint64_t grow,
+                                        const uint64_t (&vb)[QM_MAX_VCOLS], uint32_t vnull, qm_status *st = nullptr) {
+  atomicAdd(reinterpret_cast<unsigned long long *>(tp + A.w_count), 1ULL);
+  if (A.w_first >= 0) atomicMin(reinterpret_cast<unsigned long long *>(tp + A.w_first), (unsigned long long)grow);
 #pragma unroll
   for (int c = 0; c < QM_NV_BOUND(NV); ++c) {
     if (NV > QM_MAX_VCOLS && c >= A.n_vcols) break;
-    if ((vnull >> c) & 1) continue;
+    if (FT <= QM_FT_GEN && ((vnull >> c) & 1)) continue;
     const qm_vcol &vc = A.vcol[c];
     const int f = vc.flags;
-    if (f & VF_NN) atomicAdd(reinterpret_cast<unsigned long long *>(tp + (int64_t)vc.w_nn * ws), 1ULL);
-    if (vc.dtype == QM_I32 || vc.dtype == QM_I64) {
+    if (FT <= QM_FT_GEN && (f & VF_NN)) atomicAdd(reinterpret_cast<unsigned long long *>(tp + vc.w_nn), 1ULL);
+    if (FT <= QM_FT_MIX && (vc.dtype == QM_I32 || vc.dtype == QM_I64)) {
       const int64_t v = (int64_t)vb[c];
       if ((f & VF_SUM) && v != 0) {
-        uint64_t *w0 = tp + (int64_t)vc.w_sum * ws;
-        if ((local && !(f & VF_WIDE)) || (f & VF_NARROW))
-          atomicAdd(reinterpret_cast<unsigned long long *>(w0), (unsigned long long)v);
-        else add128(w0, w0 + ws, (uint64_t)v, v < 0 ? -1 : 0);
+        uint64_t *w0 = tp + vc.w_sum;
+        if (f & VF_NARROW) atomicAdd(reinterpret_cast<unsigned long long *>(w0), (unsigned long long)v);
+        else add128(w0, w0 + 1, (uint64_t)v, v < 0 ? -1 : 0);
       }
-      if (f & VF_MIN) gmin(c, tp + (int64_t)vc.w_min * ws, v);
-      if (f & VF_MAX) gmax(c, tp + (int64_t)vc.w_max * ws, v);
+      if (f & VF_MIN) atomicMin(reinterpret_cast<long long *>(tp + vc.w_min), (long long)v);
+      if (f & VF_MAX) atomicMax(reinterpret_cast<long long *>(tp + vc.w_max), (long long)v);
     } else {
       const double d = __longlong_as_double((long long)vb[c]);
-      if (f & VF_SUM) {
-        uint64_t *w0 = tp + (int64_t)vc.w_sum * ws;
-        if (FX && (f & VF_FIXED)) {
+      if (FT == QM_FT_SUM || (f & VF_SUM)) {
+        uint64_t *w0 = tp + vc.w_sum;
+        if (FT == QM_FT_FULL && (f & VF_FIXED)) {
           uint64_t lo;
           int64_t hi;
           uint32_t nf;
           bool stale = false;
           fx_cell(vc, d, lo, hi, nf, stale);
           if (stale && st) set_error(st, QM_DEV_STALE);
-          if (lo != 0 || hi != 0) add128(w0, w0 + ws, lo, hi);
-          if (nf) atomicOr(reinterpret_cast<unsigned long long *>(tp + (int64_t)vc.w_nf * ws), (unsigned long long)nf);
-        } else if (vc.split != 0.0) {
-          split_add(w0, w0 + ws, d, vc.split);
+          if (lo != 0 || hi != 0) add128(w0, w0 + 1, lo, hi);
+          if (nf) atomicOr(reinterpret_cast<unsigned long long *>(tp + vc.w_nf), (unsigned long long)nf);
+        } else if (FT >= QM_FT_MIX || vc.split != 0.0) {
+          split_add(w0, w0 + 1, d, vc.split);
         } else {
-          fsum_add(w0, w0 + ws, d, 0.0);
+          fsum_add(w0, w0 + 1, d, 0.0);
         }
       }
-      if ((f & (VF_MIN | VF_MAX)) && !isnan(d)) {  // NaN never wins '<' / '>'
-        const int64_t o = f2ord(d == 0.0 ? 0.0 : d);
-        if (f & VF_MIN) gmin(c, tp + (int64_t)vc.w_min * ws, o);
-        if (f & VF_MAX) gmax(c, tp + (int64_t)vc.w_max * ws, o);
+      if (FT <= QM_FT_MIX) {
+        if ((f & (VF_MIN | VF_MAX)) && !isnan(d)) {  // NaN never wins '<' / '>'
+          const int64_t o = f2ord(d == 0.0 ? 0.0 : d);
+          if (f & VF_MIN) atomicMin(reinterpret_cast<long long *>(tp + vc.w_min), (long long)o);
+          if (f & VF_MAX) atomicMax(reinterpret_cast<long long *>(tp + vc.w_max), (long long)o);
+        }
+        if ((f & VF_ZERO) && d == 0.0)
+          atomicMin(reinterpret_cast<unsigned long long *>(tp + vc.w_zero),
+                    (unsigned long long)((grow << 1) | (vb[c] >> 63)));
       }
-      if ((f & VF_ZERO) && d == 0.0) upd_min_u64(tp + (int64_t)vc.w_zero * ws, (grow << 1) | (vb[c] >> 63), local);
     }
   }
 }
 
-// Equal-slot merge for a drain round: lanes in `peers` (same block-local
-// slot, mask `lmask` = every lane taking this path) sum their additive
-// contributions through the warp's shared scratch, and the group leader adds
-// them once; MIN / MAX / FIRST stay per lane (64-bit min/max atomics resolve
-// conflicts in hardware, and most are skipped by the read test).
-template <int NV = QM_NV_ANY, bool FX = true>
-__device__ __forceinline__ void agg_row_merged(const qm_aggspec &A, uint64_t *tp, int L, unsigned lmask, unsigned peers,
-                                               int lane, uint64_t grow, const uint64_t (&vb)[QM_MAX_VCOLS],
-                                               uint32_t vnull, uint64_t *scr, qm_status *st = nullptr) {
-  const bool leader = lane == __ffs(peers) - 1;
-  if (leader) atomicAdd(reinterpret_cast<unsigned long long *>(tp + (int64_t)A.w_count * L), (unsigned long long)__popc(peers));
-  if (A.w_first >= 0) min_u64(tp + (int64_t)A.w_first * L, grow);
-  const int nv = NV > QM_MAX_VCOLS ? A.n_vcols : NV;
+// ---- block-local words ---------------------------------------------------------
+// Shared memory has native 32-bit atomics only; a 64-bit integer or double
+// atomic is a compare-and-swap loop (measured per warp and SM: 18 cycles on
+// 4,096 random slots, 24 on 512, 56 on 64, 111 on 16, against 1 for a 32-bit
+// add and 4 for two limbs with a carry), and merging equal slots first costs
+// more than it saves (__match_any_sync: 53-62 cycles on random slots).  So
+// the words of a block-local table that take an add per row are split into
+// 32-bit limbs: word w of slot s has its low limb at lw32(w)[s] and its high
+// limb at lw32(w)[L + s], where lw32(w) is the word's 8 * L bytes.
+//   COUNT, NN       low limb only (a block counts fewer than 2^32 rows)
+//   FIRST           low limb: the row within this launch (32-bit in the queue)
+//   integer sums    two limbs a 64-bit word, carries passed on
+//   split float sum two 64-bit integers in limbs (local_fsum)
+//   fixed-point sum 128 bits in limbs
+// MIN / MAX / FZERO (read first: most rows change nothing), FNF and the
+// TwoSum words of a column without statistics stay 64-bit words at lw[w * L + s].
+// Against 64-bit atomics with equal slots merged through __match_any_sync
+// (whole queries, B200): 200M rows into 16 groups 1.23 -> 0.76 ms, 5M rows
+// without GROUP BY 0.29 -> 0.17 ms, 100M events into 65,536 groups 0.78 ->
+// 0.71 ms.
+__device__ __forceinline__ uint32_t *limb(uint64_t *lw, int L, int w, int s) {
+  return reinterpret_cast<uint32_t *>(lw + (int64_t)w * L) + s;
+}
+
+// p[0] += v (64-bit, limbs p[0] and p[L]); returns the carry out of bit 63.
+__device__ __forceinline__ uint32_t limb_add64(uint32_t *p, int L, uint64_t v) {
+  const uint32_t v0 = (uint32_t)v;
+  uint64_t v1 = v >> 32;
+  if (v0) {
+    const uint32_t o = atomicAdd(p, v0);
+    v1 += (o + v0) < o ? 1 : 0;
+  }
+  uint32_t carry = (uint32_t)(v1 >> 32);
+  const uint32_t h = (uint32_t)v1;
+  if (h) {
+    const uint32_t o = atomicAdd(p + L, h);
+    carry += (o + h) < o ? 1 : 0;
+  }
+  return carry;
+}
+
+// As limb_add64 where the sum is read modulo 2^64 (no carry out).
+__device__ __forceinline__ void limb_add64w(uint32_t *p, int L, uint64_t v) {
+  // (adding a zero limb costs less than the branch around it)
+  const uint32_t v0 = (uint32_t)v;
+  const uint32_t o = atomicAdd(p, v0);
+  atomicAdd(p + L, (uint32_t)(v >> 32) + ((o + v0) < o ? 1u : 0u));
+}
+
+__device__ __forceinline__ void limb_add128(uint32_t *p, int L, uint64_t lo, int64_t hi) {
+  hi += (int64_t)limb_add64(p, L, lo);
+  if (hi != 0) limb_add64w(p + 2 * L, L, (uint64_t)hi);
+}
+
+// A cell of a split column added to its block-local integers.  x + sa rounds
+// x to a multiple of ga; the bits of that sum less the bits of sa are the
+// multiple itself, an integer below 2^(62 - b) for a table of fewer than
+// 2^(b - 1) rows, so the integers of a slot add up without overflow and
+// exactly, in any order.  The rest (at most ga / 2) goes to the second
+// integer in units of gb the same way; what is left below that (only cells
+// smaller than 2^(2b - 73) of the column's bound have any: 2^-17 of it at 100M
+// rows, 2^-31 at 1M) is returned for the group's global low word.
+// Returns false for a cell outside the planned range (NaN, Infinity, or a
+// column rewritten after its statistics): it goes to the global words whole.
+__device__ __forceinline__ bool local_fsum(uint32_t *p, int L, const qm_vcol &vc, double x, double &rest) {
+  rest = 0.0;
+  if (!(fabs(x) < vc.lim)) return false;
+  const double ta = __dadd_rn(x, vc.sa);
+  const double xb = __dsub_rn(x, __dsub_rn(ta, vc.sa));
+  const double tb = __dadd_rn(xb, vc.sb);
+  rest = __dsub_rn(xb, __dsub_rn(tb, vc.sb));
+  limb_add64w(p, L, (uint64_t)(__double_as_longlong(ta) - __double_as_longlong(vc.sa)));
+  limb_add64w(p + 2 * L, L, (uint64_t)(__double_as_longlong(tb) - __double_as_longlong(vc.sb)));
+  return true;
+}
+
+// One row's update of block-local slot ls (key / special: its group, for the
+// rare parts of a float sum that go to the global slot).
+template <int NV = QM_NV_ANY, int FT = QM_FT_FULL>
+__device__ __forceinline__ void agg_row_local(const qm_scan_args &a, uint64_t *lw, int L, int ls, uint64_t key,
+                                              int special, uint32_t row, const uint64_t (&vb)[QM_MAX_VCOLS],
+                                              uint32_t vnull) {
+  const qm_aggspec &A = a.agg;
+  atomicAdd(limb(lw, L, A.w_count, ls), 1u);
+  if (A.w_first >= 0) atomicMin(limb(lw, L, A.w_first, ls), row);
 #pragma unroll
-  for (int c = 0; c < nv; ++c) {
+  for (int c = 0; c < QM_NV_BOUND(NV); ++c) {
+    if (NV > QM_MAX_VCOLS && c >= A.n_vcols) break;
+    if (FT <= QM_FT_GEN && ((vnull >> c) & 1)) continue;
     const qm_vcol &vc = A.vcol[c];
     const int f = vc.flags;
-    const bool valid = !((vnull >> c) & 1);
-    if (f & VF_NN) {
-      const unsigned nn = __popc(__ballot_sync(lmask, valid) & peers);
-      if (leader && nn) atomicAdd(reinterpret_cast<unsigned long long *>(tp + (int64_t)vc.w_nn * L), (unsigned long long)nn);
-    }
-    const bool isint = vc.dtype == QM_I32 || vc.dtype == QM_I64;
-    const uint64_t raw = vget<NV>(vb, c);
-    if (f & VF_SUM) {
-      uint64_t *w0 = tp + (int64_t)vc.w_sum * L;
-      if (isint) {
-        scr[lane] = valid ? raw : 0;
-        __syncwarp(lmask);
-        if (leader) {
-          // 128-bit sum of up to 32 cells (int64 cells can carry out of 64 bits)
-          uint64_t lo = 0;
-          int64_t hi = 0;
-          for (unsigned m = peers; m; m &= m - 1) {
-            const int64_t x = (int64_t)scr[__ffs(m) - 1];
-            const uint64_t nlo = lo + (uint64_t)x;
-            hi += (x < 0 ? -1 : 0) + (nlo < lo ? 1 : 0);
-            lo = nlo;
-          }
-          if (f & VF_WIDE) {
-            if (lo != 0 || hi != 0) add128(w0, w0 + L, lo, hi);
-          } else if (lo != 0) {
-            atomicAdd(reinterpret_cast<unsigned long long *>(w0), (unsigned long long)lo);  // int32 cells: fits
-          }
-        }
-        __syncwarp(lmask);
-      } else if (FX && (f & VF_FIXED)) {
-        const double d = valid ? __longlong_as_double((long long)raw) : 0.0;
-        uint64_t lo;
-        int64_t hi;
-        uint32_t nf;
-        bool stale = false;
-        fx_cell(vc, d, lo, hi, nf, stale);
-        if (stale && st) set_error(st, QM_DEV_STALE);
-        if (nf) atomicOr(reinterpret_cast<unsigned long long *>(tp + (int64_t)vc.w_nf * L), (unsigned long long)nf);
-        scr[lane] = lo;
-        scr[32 + lane] = (uint64_t)hi;
-        __syncwarp(lmask);
-        if (leader) {
-          uint64_t slo = 0;
-          int64_t shi = 0;
-          for (unsigned m = peers; m; m &= m - 1) {
-            const int src = __ffs(m) - 1;
-            const uint64_t nlo = slo + scr[src];
-            shi += (int64_t)scr[32 + src] + (nlo < slo ? 1 : 0);
-            slo = nlo;
-          }
-          if (slo != 0 || shi != 0) add128(w0, w0 + L, slo, shi);
-        }
-        __syncwarp(lmask);
-      } else {
-        const double d = valid ? __longlong_as_double((long long)raw) : 0.0;
-        double h, l;
-        if (vc.split != 0.0) split_parts(d, vc.split, h, l);
-        else {
-          h = d;
-          l = 0.0;
-        }
-        scr[lane] = (uint64_t)__double_as_longlong(h);
-        scr[32 + lane] = (uint64_t)__double_as_longlong(l);
-        __syncwarp(lmask);
-        if (leader) {
-          if (vc.split != 0.0) {
-            double sh = 0.0, sl = 0.0;
-            for (unsigned m = peers; m; m &= m - 1) {
-              const int src = __ffs(m) - 1;
-              sh += __longlong_as_double((long long)scr[src]);  // exact: grid multiples below split
-              sl += __longlong_as_double((long long)scr[32 + src]);
-            }
-            if (sh != 0.0) atomicAdd(reinterpret_cast<double *>(w0), sh);
-            if (sl != 0.0) atomicAdd(reinterpret_cast<double *>(w0 + L), sl);
-          } else {
-            double s = 0.0, cc = 0.0;
-            for (unsigned m = peers; m; m &= m - 1) two_sum_acc(s, cc, __longlong_as_double((long long)scr[__ffs(m) - 1]));
-            fsum_add(w0, w0 + L, s, cc);
-          }
-        }
-        __syncwarp(lmask);
+    if (FT <= QM_FT_GEN && (f & VF_NN)) atomicAdd(limb(lw, L, vc.w_nn, ls), 1u);
+    if (FT <= QM_FT_MIX && (vc.dtype == QM_I32 || vc.dtype == QM_I64)) {
+      const int64_t v = (int64_t)vb[c];
+      if (f & VF_SUM) {
+        uint32_t *p = limb(lw, L, vc.w_sum, ls);
+        if (FT <= QM_FT_GEN && (f & VF_WIDE)) limb_add128(p, L, (uint64_t)v, v < 0 ? -1 : 0);
+        else limb_add64w(p, L, (uint64_t)v);
       }
-    }
-    if (!valid) continue;
-    if (isint) {
-      const int64_t v = (int64_t)raw;
-      if (f & VF_MIN) min_i64(tp + (int64_t)vc.w_min * L, v);
-      if (f & VF_MAX) max_i64(tp + (int64_t)vc.w_max * L, v);
+      if (f & VF_MIN) min_i64(lw + (int64_t)vc.w_min * L + ls, v);
+      if (f & VF_MAX) max_i64(lw + (int64_t)vc.w_max * L + ls, v);
     } else {
-      const double d = __longlong_as_double((long long)raw);
-      if ((f & (VF_MIN | VF_MAX)) && !isnan(d)) {
-        const int64_t o = f2ord(d == 0.0 ? 0.0 : d);
-        if (f & VF_MIN) min_i64(tp + (int64_t)vc.w_min * L, o);
-        if (f & VF_MAX) max_i64(tp + (int64_t)vc.w_max * L, o);
+      const double d = __longlong_as_double((long long)vb[c]);
+      if (FT == QM_FT_SUM || (f & VF_SUM)) {
+        if (FT == QM_FT_FULL && (f & VF_FIXED)) {
+          uint64_t lo;
+          int64_t hi;
+          uint32_t nf;
+          bool stale = false;
+          fx_cell(vc, d, lo, hi, nf, stale);
+          if (stale) set_error(a.status, QM_DEV_STALE);
+          limb_add128(limb(lw, L, vc.w_sum, ls), L, lo, hi);
+          if (nf) atomicOr(reinterpret_cast<unsigned long long *>(lw + (int64_t)vc.w_nf * L + ls), (unsigned long long)nf);
+        } else if (FT >= QM_FT_MIX || vc.split != 0.0) {
+          double rest;
+          const bool in = local_fsum(limb(lw, L, vc.w_sum, ls), L, vc, d, rest);
+          if (!in || rest != 0.0) {
+            const int64_t gs = global_slot(a, key, special);
+            if (gs >= 0) {
+              uint64_t *w0 = a.table + gs * a.stride + 1 + vc.w_sum;
+              if (in) atomicAdd(reinterpret_cast<double *>(w0 + 1), rest);
+              else split_add(w0, w0 + 1, d, vc.split);
+            }
+          }
+        } else {
+          uint64_t *w0 = lw + (int64_t)vc.w_sum * L + ls;
+          fsum_add(w0, w0 + L, d, 0.0);
+        }
       }
-      if ((f & VF_ZERO) && d == 0.0) min_u64(tp + (int64_t)vc.w_zero * L, (grow << 1) | (raw >> 63));
+      if (FT <= QM_FT_MIX) {
+        if ((f & (VF_MIN | VF_MAX)) && !isnan(d)) {  // NaN never wins '<' / '>'
+          const int64_t o = f2ord(d == 0.0 ? 0.0 : d);
+          if (f & VF_MIN) min_i64(lw + (int64_t)vc.w_min * L + ls, o);
+          if (f & VF_MAX) max_i64(lw + (int64_t)vc.w_max * L + ls, o);
+        }
+        if ((f & VF_ZERO) && d == 0.0)
+          min_u64(lw + (int64_t)vc.w_zero * L + ls, (((uint64_t)(a.row_offset) + row) << 1) | (vb[c] >> 63));
+      }
     }
   }
 }
 
 // Gather a row's value cells (float32 widened to double, as JS numbers).
-template <int NV = QM_NV_ANY>
+template <int NV = QM_NV_ANY, int FT = QM_FT_FULL>
 __device__ __forceinline__ void gather_values(const qm_aggspec &A, int64_t row, uint64_t (&vb)[QM_MAX_VCOLS],
                                               uint32_t &vnull) {
   vnull = 0;
@@ -1237,15 +1244,16 @@ __device__ __forceinline__ void gather_values(const qm_aggspec &A, int64_t row, 
     vb[c] = 0;
     if (c < QM_NV_BOUND(NV) && (NV <= QM_MAX_VCOLS || c < A.n_vcols)) {
       const qm_vcol &vc = A.vcol[c];
-      if (cell_null(vc.nulls, row)) vnull |= 1u << c;
-      else if (vc.dtype == QM_I32 || vc.dtype == QM_I64) vb[c] = (uint64_t)ld_int(vc.data, vc.dtype, row);
+      if (FT <= QM_FT_GEN && cell_null(vc.nulls, row)) vnull |= 1u << c;
+      else if (FT <= QM_FT_MIX && (vc.dtype == QM_I32 || vc.dtype == QM_I64)) vb[c] = (uint64_t)ld_int(vc.data, vc.dtype, row);
       else vb[c] = (uint64_t)__double_as_longlong(ld_flt(vc.data, vc.dtype, row));
     }
   }
 }
 
-// Merge one block-local slot (words at lp[w * L]) into global slot words gp.
-__device__ __forceinline__ void merge_local(const qm_aggspec &A, const uint64_t *lp, int L, uint64_t *gp) {
+// Merge one block-local slot of a deduplicating plan (words in the global
+// table's form, word w at lp[w * L]) into global slot words gp.
+__device__ __forceinline__ void merge_raw(const qm_aggspec &A, const uint64_t *lp, int L, uint64_t *gp) {
   for (int i = 0; i < A.n_accs; ++i) {
     const qm_acc ac = A.acc[i];
     const uint64_t v0 = lp[(int64_t)ac.word * L];
@@ -1293,6 +1301,178 @@ __device__ __forceinline__ void merge_local(const qm_aggspec &A, const uint64_t 
   }
 }
 
+// The value of one accumulator of block-local slot s (agg_row_local's words):
+// v0, v1 as 64-bit integers (split sums: the two integers; FIRST: the row
+// within the launch).
+__device__ __forceinline__ void local_load(const qm_aggspec &A, const qm_acc &ac, uint64_t *lw, int L, int s,
+                                           uint64_t &v0, uint64_t &v1) {
+  const uint32_t *p = limb(lw, L, ac.word, s);
+  v1 = 0;
+  switch (ac.kind) {
+    case QA_COUNT:
+    case QA_NN:
+    case QA_FIRST: v0 = p[0]; break;
+    case QA_ISUM:
+    case QA_FSUM:
+      if (ac.kind == QA_FSUM && !(A.vcol[ac.vcol].flags & VF_FIXED) && A.vcol[ac.vcol].split == 0.0) {
+        v0 = lw[(int64_t)ac.word * L + s];
+        v1 = lw[(int64_t)(ac.word + 1) * L + s];
+      } else {
+        v0 = p[0] | (uint64_t)p[L] << 32;
+        v1 = p[2 * L] | (uint64_t)p[3 * L] << 32;
+        if (ac.kind == QA_ISUM && !ac.wide) v1 = 0;
+      }
+      break;
+    default: v0 = lw[(int64_t)ac.word * L + s];
+  }
+}
+
+// (v0, v1) of another copy of the slot folded into this one's.
+__device__ __forceinline__ void local_fold(const qm_aggspec &A, const qm_acc &ac, uint64_t &v0, uint64_t &v1,
+                                           uint64_t x0, uint64_t x1) {
+  switch (ac.kind) {
+    case QA_COUNT:
+    case QA_NN: v0 += x0; break;
+    case QA_FIRST:
+    case QA_FZERO: v0 = min(v0, x0); break;
+    case QA_FNF: v0 |= x0; break;
+    case QA_IMIN:
+    case QA_FMIN: v0 = (uint64_t)min((int64_t)v0, (int64_t)x0); break;
+    case QA_IMAX:
+    case QA_FMAX: v0 = (uint64_t)max((int64_t)v0, (int64_t)x0); break;
+    case QA_ISUM: {
+      const uint64_t n = v0 + x0;
+      v1 += x1 + (n < v0 ? 1 : 0);
+      v0 = n;
+      break;
+    }
+    case QA_FSUM:
+      if (A.vcol[ac.vcol].flags & VF_FIXED) {
+        const uint64_t n = v0 + x0;
+        v1 += x1 + (n < v0 ? 1 : 0);
+        v0 = n;
+      } else if (A.vcol[ac.vcol].split != 0.0) {
+        v0 += x0;
+        v1 += x1;
+      } else {
+        double s = __longlong_as_double((long long)v0);
+        double c = __longlong_as_double((long long)v1) + __longlong_as_double((long long)x1);
+        two_sum_acc(s, c, __longlong_as_double((long long)x0));
+        v0 = (uint64_t)__double_as_longlong(s);
+        v1 = (uint64_t)__double_as_longlong(c);
+      }
+      break;
+  }
+}
+
+// A split sum's two integers as the global table's double words: hi the
+// multiple of ulp(split) nearest the first, lo the rest.
+__device__ __forceinline__ void split_words(const qm_vcol &vc, int64_t ai, int64_t bi, double &hi, double &lo) {
+  const int64_t h = (ai + ((int64_t)1 << vc.lsh >> 1)) >> vc.lsh;
+  const int64_t r = ai - (h << vc.lsh);
+  hi = (double)h * (vc.ga * (double)((int64_t)1 << vc.lsh));  // |h| < 2^53: exact
+  lo = (double)r * vc.ga + (double)bi * vc.gb;
+}
+
+// One accumulator's value (local_load) into global slot words gp.
+__device__ __forceinline__ void merge_value(const qm_aggspec &A, const qm_acc &ac, uint64_t v0, uint64_t v1, uint64_t *gp,
+                                            int64_t row_offset) {
+  uint64_t *g0 = gp + ac.word, *g1 = gp + ac.word + 1;
+  switch (ac.kind) {
+    case QA_COUNT:
+    case QA_NN:
+      if (v0) atomicAdd(reinterpret_cast<unsigned long long *>(g0), (unsigned long long)v0);
+      break;
+    case QA_FIRST:  // an occupied slot has a row
+      atomicMin(reinterpret_cast<unsigned long long *>(g0), (unsigned long long)row_offset + (unsigned long long)v0);
+      break;
+    case QA_FZERO:
+      if (v0 != ~0ULL) atomicMin(reinterpret_cast<unsigned long long *>(g0), (unsigned long long)v0);
+      break;
+    case QA_ISUM:
+      if (ac.wide) add128(g0, g1, v0, (int64_t)v1);
+      else if (v0 && ac.narrow) atomicAdd(reinterpret_cast<unsigned long long *>(g0), (unsigned long long)v0);
+      else if (v0) add128(g0, g1, v0, (int64_t)v0 < 0 ? -1 : 0);
+      break;
+    case QA_FNF:
+      if (v0) atomicOr(reinterpret_cast<unsigned long long *>(g0), (unsigned long long)v0);
+      break;
+    case QA_FSUM:
+      if (A.vcol[ac.vcol].flags & VF_FIXED) {
+        if (v0 || v1) add128(g0, g1, v0, (int64_t)v1);
+      } else if (A.vcol[ac.vcol].split != 0.0) {
+        double h, l;
+        split_words(A.vcol[ac.vcol], (int64_t)v0, (int64_t)v1, h, l);
+        if (h != 0.0) atomicAdd(reinterpret_cast<double *>(g0), h);
+        if (l != 0.0) atomicAdd(reinterpret_cast<double *>(g1), l);
+      } else {
+        fsum_add(g0, g1, __longlong_as_double((long long)v0), __longlong_as_double((long long)v1));
+      }
+      break;
+    case QA_IMIN:
+    case QA_FMIN:
+      if ((int64_t)v0 != (int64_t)A.init[ac.word]) atomicMin(reinterpret_cast<long long *>(g0), (long long)v0);
+      break;
+    case QA_IMAX:
+    case QA_FMAX:
+      if ((int64_t)v0 != (int64_t)A.init[ac.word]) atomicMax(reinterpret_cast<long long *>(g0), (long long)v0);
+      break;
+  }
+}
+
+// Block-local slot s (agg_row_local's words) into global slot words gp.
+__device__ __forceinline__ void merge_local(const qm_aggspec &A, uint64_t *lw, int L, int s, uint64_t *gp,
+                                            int64_t row_offset) {
+  for (int i = 0; i < A.n_accs; ++i) {
+    const qm_acc ac = A.acc[i];
+    uint64_t v0, v1;
+    local_load(A, ac, lw, L, s, v0, v1);
+    merge_value(A, ac, v0, v1, gp, row_offset);
+  }
+}
+
+// A whole block's local table into the global table (every thread of the
+// block calls this after a barrier).  With copies, the lanes of a copy group
+// fold theirs by shuffles first, so the block adds once per slot and word.
+__device__ __forceinline__ void merge_block(const qm_scan_args &a, const uint64_t *lkeys, uint64_t *lw) {
+  const qm_aggspec &A = a.agg;
+  const int L = a.local_slots;
+  if (a.dedupe) {
+    for (int s = threadIdx.x; s < L; s += blockDim.x) {
+      if (lw[(int64_t)A.w_count * L + s] == 0) continue;
+      const int64_t gs = a.local_hash ? global_slot(a, lkeys[s], 0) : s;
+      if (gs >= 0) merge_raw(A, lw + s, L, a.table + gs * a.stride + 1);
+    }
+    return;
+  }
+  if (a.local_rep == 0) {
+    for (int s = threadIdx.x; s < L; s += blockDim.x) {
+      if (*limb(lw, L, A.w_count, s) == 0) continue;
+      const int64_t gs = a.local_hash ? global_slot(a, lkeys[s], 0) : s;
+      if (gs >= 0) merge_local(A, lw, L, s, a.table + gs * a.stride + 1, a.row_offset);
+    }
+    return;
+  }
+  const int copies = 1 << a.local_rep;
+  for (int s0 = threadIdx.x & ~31; s0 < L; s0 += blockDim.x) {  // whole warps: L is a multiple of the copies, not of 32
+    const int s = s0 + (threadIdx.x & 31);
+    const bool in = s < L;
+    unsigned any = __ballot_sync(QM_FULL, in && *limb(lw, L, A.w_count, s) != 0);
+    any = (any >> ((threadIdx.x & 31) & ~(copies - 1))) & (copies == 32 ? QM_FULL : (1u << copies) - 1u);
+    uint64_t *gp = a.table + (int64_t)(s >> a.local_rep) * a.stride + 1;
+    for (int i = 0; i < A.n_accs; ++i) {
+      const qm_acc ac = A.acc[i];
+      uint64_t v0 = 0, v1 = 0;
+      if (in) local_load(A, ac, lw, L, s, v0, v1);
+      for (int o = copies >> 1; o; o >>= 1) {
+        const uint64_t x0 = __shfl_xor_sync(QM_FULL, v0, o), x1 = __shfl_xor_sync(QM_FULL, v1, o);
+        local_fold(A, ac, v0, v1, x0, x1);
+      }
+      if (any && in && (s & (copies - 1)) == 0) merge_value(A, ac, v0, v1, gp, a.row_offset);
+    }
+  }
+}
+
 // Fold block-local slot words src[w * L] into dst[w * L] (both in this
 // block's shared memory, no other writer): the per-warp copies of a private
 // table collapse into one before the global merge.
@@ -1329,13 +1509,13 @@ __device__ __forceinline__ void merge_plain(const qm_aggspec &A, uint64_t *dst, 
   }
 }
 
-// Applies one survivor per lane (key word, special flag, global row and
-// gathered cells; lanes with active = false sit out) to the block-local
-// table or else the global table.
-template <int DD = 2, int NV = QM_NV_ANY, bool FX = true>
+// Applies one survivor per lane (key word, special flag, row within the
+// launch and gathered cells; lanes with active = false sit out) to the
+// block-local table or else the global table.
+template <int DD = 2, int NV = QM_NV_ANY, int FT = QM_FT_FULL, int LM = QM_LM_ANY>
 __device__ __forceinline__ void drain_apply(const qm_scan_args &a, uint64_t *lkeys, uint64_t *lw, int L, int *l_used,
-                                            int lane, bool active, uint64_t key, int special, uint64_t grow,
-                                            const uint64_t (&vb)[QM_MAX_VCOLS], uint32_t vnull, uint64_t *scr) {
+                                            int lane, bool active, uint64_t key, int special, uint32_t row,
+                                            const uint64_t (&vb)[QM_MAX_VCOLS], uint32_t vnull) {
   const qm_aggspec &A = a.agg;
   if (DD == 2 ? a.dedupe != 0 : DD == 1) {
     const unsigned act = __ballot_sync(QM_FULL, active);
@@ -1362,45 +1542,61 @@ __device__ __forceinline__ void drain_apply(const qm_scan_args &a, uint64_t *lke
       }
     }
     const int iters = (int)__reduce_max_sync(act, (unsigned)__popc(peers)) - 1;
-    apply_row<FX>(A, tp, ws, local, act, peers, iters, lane, grow, vb, vnull, local && a.priv, FX ? a.status : nullptr);
+    apply_row<FT == QM_FT_FULL>(A, tp, ws, local, act, peers, iters, lane, (uint64_t)a.row_offset + row, vb, vnull,
+                                local && a.priv, FT == QM_FT_FULL ? a.status : nullptr);
+    return;
+  }
+  if (LM == QM_LM_DIRECT) {
+    if (active) {
+      const int64_t s = global_slot(a, key, special);
+      if (s >= 0)
+        agg_row_local<NV, FT>(a, lw, L, ((int)s << a.local_rep) | (lane & ((1 << a.local_rep) - 1)), key, special, row, vb,
+                              vnull);
+    }
+    __syncwarp();
     return;
   }
   int ls = -1;
-  if (active && L > 0) {
-    if (!a.local_hash) ls = (int)global_slot(a, key, special);
-    else if (special == 0) ls = local_find(lkeys, L, key, l_used);
+  bool global = active;
+  if (L > 0 && active) {
+    if (!a.local_hash) {
+      const int64_t s = global_slot(a, key, special);
+      global = false;
+      if (s >= 0) ls = ((int)s << a.local_rep) | (lane & ((1 << a.local_rep) - 1));
+    } else if (special == 0) {
+      ls = local_find(lkeys, L, key, l_used);
+      global = ls < 0;
+    }
   }
-  const bool loc = active && ls >= 0;
-  const unsigned lmask = __ballot_sync(QM_FULL, loc);
-  unsigned peers = 0;
-  if (loc) peers = __match_any_sync(lmask, ls);
-  const bool merge = __any_sync(QM_FULL, (peers & (peers - 1)) != 0);
-  if (loc) {
-    if (merge) agg_row_merged<NV, FX>(A, lw + ls, L, lmask, peers, lane, grow, vb, vnull, scr, FX ? a.status : nullptr);
-    else agg_row<NV, FX>(A, lw + ls, L, true, grow, vb, vnull, FX ? a.status : nullptr);
-  } else if (active && !(L > 0 && !a.local_hash)) {
-    const int64_t gs = global_slot(a, key, special);
-    if (gs >= 0) agg_row<NV, FX>(A, a.table + gs * a.stride + 1, 1, false, grow, vb, vnull, FX ? a.status : nullptr);
-  }
+  // the lanes leave the probe loops at different steps: meet again before the
+  // updates, or each lane walks them alone
+  __syncwarp();
+  if (ls >= 0) agg_row_local<NV, FT>(a, lw, L, ls, key, special, row, vb, vnull);
+  __syncwarp();
+  int64_t gs = -1;
+  if (global) gs = global_slot(a, key, special);
+  __syncwarp();
+  if (gs >= 0)
+    agg_row<NV, FT>(A, a.table + gs * a.stride + 1, (uint64_t)a.row_offset + row, vb, vnull,
+                    FT == QM_FT_FULL ? a.status : nullptr);
 }
 
 // Aggregates one survivor per lane (lanes with active = false sit out):
 // gathers its key and value cells, then drain_apply.
 // DD: 0 / 1 = the plan's dedupe flag fixed at compile time (separate kernels
 // keep each path's registers and code apart), 2 = read it from the plan.
-template <int DD = 2, int NV = QM_NV_ANY, int KK = QM_KK_ANY, bool FX = true>
+template <int DD = 2, int NV = QM_NV_ANY, int KK = QM_KK_ANY, int FT = QM_FT_FULL, int LM = QM_LM_ANY>
 __device__ __forceinline__ void drain_round_any(const qm_scan_args &a, uint64_t *lkeys, uint64_t *lw, int L,
-                                                int *l_used, int lane, bool active, int64_t row, uint64_t *scr) {
-  uint64_t grow = 0, key = 0;
+                                                int *l_used, int lane, bool active, int64_t row) {
+  uint64_t key = 0;
   int special = 0;
   uint64_t vb[QM_MAX_VCOLS];
   uint32_t vnull = 0;
   if (active) {
-    grow = (uint64_t)(a.row_offset + row);
     key = row_key<KK>(a.key, row, special);
-    gather_values<NV>(a.agg, row, vb, vnull);
+    gather_values<NV, FT>(a.agg, row, vb, vnull);
   }
-  drain_apply<DD, NV, FX>(a, lkeys, lw, L, l_used, lane, active, key, special, grow, vb, vnull, scr);
+  drain_apply<DD, NV, FT, LM>(a, lkeys, lw, L, l_used, lane, active, key, special, (uint32_t)row, vb, vnull);
 }
 
 

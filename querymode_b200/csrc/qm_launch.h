@@ -11,11 +11,13 @@
 
 // Scan kernels specialised for N = 0..QM_SPEC_NV_MAX value columns
 // (qm_scan_nvN.cu): dynamic shared memory limit of each, and the launch of
-// the one for (dedupe flag, key kind QM_KK_*).
+// the one for (dedupe flag, key kind QM_KK_*, value features QM_FT_*, row
+// placement QM_LM_*), or of the least general one that covers it.
 #define QM_SPEC_NV_MAX 4
 #define QM_DECL_SPEC(N)                                                                        \
   cudaError_t qm_scan_nv##N##_attr(int max_smem);                                           \
-  cudaError_t qm_scan_nv##N##_launch(const qm_scan_args &a, int dd, int kk, int blocks, size_t smem, \
+  cudaError_t qm_scan_nv##N##_launch(const qm_scan_args &a, int dd, int kk, int ft, int lm, int blocks, \
+                                     size_t smem, \
                                      cudaStream_t st);
 QM_DECL_SPEC(0)
 QM_DECL_SPEC(1)

@@ -223,15 +223,22 @@ __global__ void qm_part_bases(const __grid_constant__ qm_part_spec ps) {
 
 // A partition's shared-memory table written into the group table by plain
 // stores: the block holding every record of the partition owns its slots.
-__device__ __forceinline__ void store_local(const qm_aggspec &A, const uint64_t *lp, int L, uint64_t *gp) {
+__device__ __forceinline__ void store_local(const qm_aggspec &A, uint64_t *lw, int L, int s, uint64_t *gp, bool raw,
+                                            int64_t row_offset) {
   for (int i = 0; i < A.n_accs; i++) {
     const qm_acc ac = A.acc[i];
-    const uint64_t v0 = lp[(int64_t)ac.word * L];
+    uint64_t v0, v1;
+    if (raw) {
+      v0 = lw[(int64_t)ac.word * L + s];
+      v1 = ac.kind == QA_FSUM || (ac.kind == QA_ISUM && ac.wide) ? lw[(int64_t)(ac.word + 1) * L + s] : 0;
+    } else {
+      local_load(A, ac, lw, L, s, v0, v1);
+    }
     uint64_t *g0 = gp + ac.word;
     if (ac.kind == QA_ISUM) {
       if (ac.wide) {
         g0[0] = v0;
-        g0[1] = lp[(int64_t)(ac.word + 1) * L];
+        g0[1] = v1;
       } else if (ac.narrow) {
         g0[0] = v0;
       } else {  // a 64-bit block-local sum into the 128-bit table word pair
@@ -239,8 +246,19 @@ __device__ __forceinline__ void store_local(const qm_aggspec &A, const uint64_t 
         g0[1] = (int64_t)v0 < 0 ? ~0ULL : 0ULL;
       }
     } else if (ac.kind == QA_FSUM) {
-      g0[0] = v0;
-      g0[1] = lp[(int64_t)(ac.word + 1) * L];
+      const qm_vcol &vc = A.vcol[ac.vcol];
+      if (!raw && !(vc.flags & VF_FIXED) && vc.split != 0.0) {
+        // added, not stored: rare parts of the sum went to these words already
+        double h, l;
+        split_words(vc, (int64_t)v0, (int64_t)v1, h, l);
+        if (h != 0.0) atomicAdd(reinterpret_cast<double *>(g0), h);
+        if (l != 0.0) atomicAdd(reinterpret_cast<double *>(g0 + 1), l);
+      } else {
+        g0[0] = v0;
+        g0[1] = v1;
+      }
+    } else if (ac.kind == QA_FIRST && !raw) {
+      g0[0] = (uint64_t)row_offset + v0;
     } else {
       g0[0] = v0;
     }
@@ -272,7 +290,6 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   const int hashed = ps.direct ? 0 : 1;
   uint64_t *lkeys = reinterpret_cast<uint64_t *>(smem);
   uint64_t *lw = lkeys + (hashed ? Lmax : 0);
-  uint64_t *scr = reinterpret_cast<uint64_t *>(smem + (size_t)Lmax * 8 * (hashed + A.n_words)) + warp * 64;
   const int nv = NV > QM_MAX_VCOLS ? A.n_vcols : NV;
   const int P1 = ps.parts + 1;
   const uint64_t total = ps.bases[P1];
@@ -306,6 +323,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       if (threadIdx.x == 0) {
         l_used = 0;
         P.priv = 0;
+        P.local_rep = 0;
         if (p == ps.parts) {
           P.local_slots = 0;
         } else if (ps.direct) {
@@ -353,23 +371,22 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
         for (int c = 0; c < QM_MAX_VCOLS; ++c) vb[c] = c < QM_NV_BOUND(NV) && c < nv ? w[2 + c] : 0;
         const int special = (int)((w[1] >> 32) & 0xff);
         const uint32_t vnull = (uint32_t)((w[1] >> 40) & 0xff);
-        const uint64_t grow = (uint64_t)a.row_offset + (uint32_t)w[1];
-        drain_apply<DD, NV, (NV > QM_MAX_VCOLS)>(P, lkeys, lw, L, &l_used, lane, active, w[0], special, grow, vb,
-                                                vnull, scr);
+        drain_apply<DD, NV, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, &l_used, lane, active, w[0], special, (uint32_t)w[1],
+                                                vb, vnull);
       }
       __syncthreads();
       if (L > 0) {
-        const int cw = A.w_count;
+        const bool raw = P.dedupe != 0;
         for (int s2 = threadIdx.x; s2 < L; s2 += blockDim.x) {
-          const uint64_t *lp = lw + s2;
-          if (lp[(int64_t)cw * L] == 0) continue;
+          if (raw ? lw[(int64_t)A.w_count * L + s2] == 0 : *limb(lw, L, A.w_count, s2) == 0) continue;
           if (!hashed && whole) {
-            store_local(A, lp, L, P.table + (int64_t)s2 * P.stride + 1);
+            store_local(A, lw, L, s2, P.table + (int64_t)s2 * P.stride + 1, raw, P.row_offset);
             continue;
           }
           const int64_t gs = hashed ? global_slot(P, lkeys[s2], 0) : s2;
           if (gs < 0) continue;
-          merge_local(A, lp, L, P.table + gs * P.stride + 1);
+          if (raw) merge_raw(A, lw + s2, L, P.table + gs * P.stride + 1);
+          else merge_local(A, lw, L, s2, P.table + gs * P.stride + 1, P.row_offset);
         }
       }
       __syncthreads();
@@ -386,7 +403,7 @@ size_t qm_part_scan_smem(int parts) {
 }
 
 size_t qm_part_agg_smem(int local_slots, int local_hash, int n_words) {
-  return (size_t)local_slots * 8 * ((local_hash ? 1 : 0) + n_words) + (size_t)(QM_SCAN_THREADS / 32) * 64 * 8;
+  return (size_t)local_slots * 8 * ((local_hash ? 1 : 0) + n_words);
 }
 
 namespace {

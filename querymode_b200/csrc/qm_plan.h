@@ -154,6 +154,13 @@ struct qm_vcol {
   int32_t fx_exp;
   int32_t w_nf;
   double fx_max;
+  // Block-local float SUM of a split column (see local_fsum): a cell below
+  // lim in magnitude is added as two 64-bit integers, in units of ga and gb,
+  // found by adding sa = 1.5 * 2^p and sb = 1.5 * 2^q (ga = 2^(p-52),
+  // gb = 2^(q-52)); ulp(split) = ga * 2^lsh.
+  double lim, sa, sb, ga, gb;
+  int32_t lsh;
+  int32_t pad2;
 };
 
 struct qm_aggspec {
@@ -256,6 +263,10 @@ struct qm_scan_args {
   int32_t max_probe;     // bound on linear probing in the global table
   int32_t priv;          // direct block-local table copied per warp: its
                          // (deduplicated) updates need no atomics
+  int32_t local_rep;     // log2 of the copies of each direct block-local slot
+                         // (lane l updates copy l mod copies; local_slots
+                         // counts the copies); 0 for hashed or deduplicated
+  int32_t pad;
   const uint32_t *zones; // zones (QM_ZONE_TILES tiles each) to scan, ascending, or null: every tile
   int64_t n_zone_tiles;  // zones: tiles covered (count of zones x QM_ZONE_TILES)
   qm_status *status;

@@ -15,7 +15,7 @@ namespace qm {
 
 struct smem_layout {
   int L;
-  size_t keys_off, words_off, queue_off, scratch_off, stage_off, stage_warp_bytes, bytes;
+  size_t keys_off, words_off, queue_off, stage_off, stage_warp_bytes, bytes;
 };
 
 // Per warp staging region: QM_STAGE_MAX_DEPTH mbarriers (32 bytes), then
@@ -29,18 +29,10 @@ __host__ __device__ inline smem_layout make_smem_layout(int local_slots, int loc
   s.words_off = kb;
   size_t wb = (size_t)local_slots * n_words * 8 * (priv ? warps : 1);  // priv: one copy per warp
   s.queue_off = (s.words_off + wb + 15) & ~(size_t)15;
-  s.scratch_off = (s.queue_off + (size_t)warps * QM_WQ * sizeof(uint32_t) + 15) & ~(size_t)15;
-  s.stage_off = (s.scratch_off + (size_t)warps * 64 * sizeof(uint64_t) + 127) & ~(size_t)127;
+  s.stage_off = (s.queue_off + (size_t)warps * QM_WQ * sizeof(uint32_t) + 127) & ~(size_t)127;
   s.stage_warp_bytes = stage_depth > 0 ? (size_t)(32 + stage_depth * stage_tile_bytes + 127) & ~(size_t)127 : 0;
   s.bytes = s.stage_off + (size_t)warps * s.stage_warp_bytes;
   return s;
-}
-
-template <bool SEL, int DD, int NV, int KK>
-__device__ __forceinline__ void drain_round(const qm_scan_args &a, uint64_t *lkeys, uint64_t *lw, int L,
-                                            int *l_used, int lane, bool active, int64_t row, uint64_t *scr) {
-  // the fixed-point sum paths only in the run-time-plan kernels
-  drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS)>(a, lkeys, lw, L, l_used, lane, active, row, scr);
 }
 
 // The fused scan.  Each warp takes tiles of QM_TILE_ROWS rows round robin,
@@ -52,8 +44,9 @@ __device__ __forceinline__ void drain_round(const qm_scan_args &a, uint64_t *lke
 // bulk async copies (lane 0 issues, an mbarrier per buffer counts the bytes)
 // while the current tile is evaluated.
 // NV / KK: the value-column count and key kind the kernel is specialised
-// for (QM_NV_ANY / QM_KK_ANY: read from the plan at run time).
-template <bool SEL, bool STAGED, int DD, int NV, int KK>
+// for (QM_NV_ANY / QM_KK_ANY: read from the plan at run time); FT / LM: what
+// its value columns need and where its rows go (QM_FT_*, QM_LM_*).
+template <bool SEL, bool STAGED, int DD, int NV, int KK, int FT, int LM>
 __global__ void __launch_bounds__(QM_SCAN_THREADS)
     qm_scan_kernel(const __grid_constant__ qm_scan_args a) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -71,7 +64,6 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   // a private (per-warp) table: this warp's copy
   uint64_t *lwm = a.priv ? lw + (int64_t)warp * L * A.n_words : lw;
   uint32_t *queue = reinterpret_cast<uint32_t *>(smem + lay.queue_off) + warp * QM_WQ;
-  uint64_t *scr = reinterpret_cast<uint64_t *>(smem + lay.scratch_off) + warp * 64;
   uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + lay.stage_off + warp * lay.stage_warp_bytes);
   uint8_t *sbuf = smem + lay.stage_off + warp * lay.stage_warp_bytes + 32;
   __shared__ int l_used;
@@ -214,7 +206,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       const int64_t row = queue[qn - 32 + lane];
       __syncwarp();
       qn -= 32;
-      drain_round<SEL, DD, NV, KK>(a, lkeys, lwm, L, &l_used, lane, true, row, scr);
+      drain_round_any<DD, NV, KK, FT, LM>(a, lkeys, lwm, L, &l_used, lane, true, row);
     }
   }
   if (STAGED && failed) {
@@ -226,7 +218,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
     const bool active = lane < qn;
     const int64_t row = active ? (int64_t)queue[lane] : 0;
     __syncwarp();
-    drain_round<SEL, DD, NV, KK>(a, lkeys, lwm, L, &l_used, lane, active, row, scr);
+    drain_round_any<DD, NV, KK, FT, LM>(a, lkeys, lwm, L, &l_used, lane, active, row);
   }
 
   if (lane == 0 && selected) atomicAdd(&blk_selected, selected);
@@ -235,8 +227,8 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
 
   // merge the block-local table into the global table
   if (L > 0) {
-    const int cw = A.w_count;
     if (a.priv) {  // fold the per-warp copies into copy 0
+      const int cw = A.w_count;
       for (int s = threadIdx.x; s < L; s += blockDim.x)
         for (int w = 1; w < warps; ++w) {
           const uint64_t *src = lw + (int64_t)w * L * A.n_words + s;
@@ -244,15 +236,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
         }
       __syncthreads();
     }
-    for (int s = threadIdx.x; s < L; s += blockDim.x) {
-      const uint64_t *lp = lw + s;
-      if (lp[(int64_t)cw * L] == 0) continue;
-      int64_t gs;
-      if (a.local_hash) gs = global_slot(a, lkeys[s], 0);
-      else gs = s;
-      if (gs < 0) continue;
-      merge_local(A, lp, L, a.table + gs * a.stride + 1);
-    }
+    merge_block(a, lkeys, lw);
   }
 }
 
