@@ -1593,10 +1593,12 @@ int post_aggregate(qm_ctx *ctx, const Plan &pl, const qm_outspec &O, int64_t G, 
       const int64_t held = std::min(k, G);
       if ((rc = ensure(ctx, ctx->post_idx2, std::max<int64_t>(held, 1) * 4))) return rc;
       if (G > 0xffffffffLL) return set_err(ctx, QM_ERR_UNSUPPORTED, "ORDER BY over more than 2^32 groups");
+      if ((rc = ensure(ctx, ctx->post_temp, qm_topk_temp_bytes(G, k, wide)))) return rc;
+      int launched = 0;
       CK(qm_launch_topk((const uint32_t *)ctx->post_last.p, (const uint64_t *)ctx->post_hi.p,
-                        (const uint64_t *)ctx->post_lo.p, G, k, (uint32_t *)ctx->post_idx.p,
-                        (uint32_t *)ctx->post_idx2.p, ctx->stream));
-      ctx->launches++;
+                        (const uint64_t *)ctx->post_lo.p, wide, G, k, (uint32_t *)ctx->post_idx.p,
+                        (uint32_t *)ctx->post_idx2.p, ctx->post_temp.p, ctx->sm_count, &launched, ctx->stream));
+      ctx->launches += launched;
       idx = (const uint32_t *)ctx->post_idx2.p;
       first = std::min(pl.post_offset, held);
       n = held - first;

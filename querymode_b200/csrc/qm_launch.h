@@ -101,8 +101,11 @@ cudaError_t qm_launch_sort_keys(const unsigned char *data, const uint32_t *nulls
 cudaError_t qm_stable_sort_rows(const uint32_t *last, const uint64_t *hi, const uint64_t *lo, bool wide, int64_t G,
                                 uint32_t *idx, uint32_t *idx2, uint64_t *k1, uint64_t *k2, uint32_t *l1, uint32_t *l2,
                                 void *temp, size_t *temp_bytes, int sm_count, cudaStream_t st);
-cudaError_t qm_launch_topk(const uint32_t *last, const uint64_t *hi, const uint64_t *lo, int64_t G, int64_t k,
-                           uint32_t *heap, uint32_t *out, cudaStream_t st);
+// Top k (heap: G entries, for the serial heap; temp: qm_topk_temp_bytes, 0
+// where only that heap runs).  *launches: kernels launched.
+size_t qm_topk_temp_bytes(int64_t G, int64_t k, bool wide);
+cudaError_t qm_launch_topk(const uint32_t *last, const uint64_t *hi, const uint64_t *lo, bool wide, int64_t G, int64_t k,
+                           uint32_t *heap, uint32_t *out, void *temp, int sm_count, int *launches, cudaStream_t st);
 // rows idx[first + j] (or first + j when idx is null), j < n
 cudaError_t qm_launch_gather_rows(const unsigned char *src, const qm_outspec &O, const qm_outspec &O2,
                                   const uint32_t *idx, int64_t first, int64_t n, unsigned char *dst, int sm_count,
