@@ -201,13 +201,15 @@ typedef struct {
   int64_t rows_selected;
   int64_t groups;
   int64_t bytes_scanned;  /* algorithmic: rows x widths of referenced columns */
-  double device_ms;       /* CUDA-event time of the device work of the run  */
+  double device_ms;       /* time of the device work of the run (CUDA events;
+                             the GPU's own timer where one block finishes the
+                             result)                                         */
   int32_t strategy;       /* 0 direct-mapped, 1 block-local + global hash,
                              2 global hash only, 3 hash-partitioned          */
   int32_t table_capacity; /* log2 of the group table's slot count           */
   int32_t retries;        /* table regrowths after a capacity overflow      */
   int32_t launches;       /* kernels of this library launched by the run   */
-  double scan_ms;         /* CUDA-event time of the fused scan kernel(s)    */
+  double scan_ms;         /* ... of the fused scan kernel(s)                */
 } qm_stats;
 
 /* Launch-shape knobs of the fused scan kernel, chosen by the autotuner

@@ -228,6 +228,7 @@ struct qm_ctx {
   DevBuf masks, counts, offsets, sel_out, sel_in;
   DevBuf agg_spare;  // group table of a destroyed qm_agg, reused by the next one
   DevBuf fbits, fcounts, franks;  // first-row bitmap, its popcounts and prefix sums
+  DevBuf tail;                    // small results (qm_tail): times, then NULL bytes
   DevBuf perm;                    // slot of each ranked output row (large results)
   DevBuf zstat, zones;           // zone-map statistics pass; the kept zones of a query
   DevBuf part_counts, part_offsets, part_bases, part_records;  // partitioned aggregation
@@ -1114,8 +1115,10 @@ std::map<std::tuple<int, int, size_t>, int> g_occ;
 // lane's larger launch.
 std::map<std::pair<int, int>, size_t> g_class_attr;
 
+// The launch's blocks and its rows per lane (a.lane_rows, from a.n and a.sel).
 // cap: blocks per SM for this launch unless the context's tuning sets them.
-int scan_blocks(qm_ctx *ctx, size_t smem, int64_t n, bool staged, int cap = 0) {
+int scan_shape(qm_ctx *ctx, qm_scan_args &a, size_t smem, bool staged, int cap = 0) {
+  const int64_t n = a.n;
   int bps = 1;
   {
     std::lock_guard<std::mutex> lk(g_cfg_mu);
@@ -1136,11 +1139,21 @@ int scan_blocks(qm_ctx *ctx, size_t smem, int64_t n, bool staged, int cap = 0) {
   } else if (cap > 0 && cap < bps) {
     bps = cap;
   }
-  int64_t tiles = (n + QM_TILE_ROWS - 1) / QM_TILE_ROWS;
-  int64_t warps = QM_SCAN_THREADS / 32;
-  int64_t need = (tiles + warps - 1) / warps;
-  int64_t blocks = std::min<int64_t>((int64_t)ctx->sm_count * bps, std::max<int64_t>(need, 1));
-  return (int)blocks;
+  const int64_t warps = QM_SCAN_THREADS / 32, most = (int64_t)ctx->sm_count * bps;
+  // A tile of 256 rows is drained 32 rows at a time, one after another: while
+  // warps would stay idle, shorter tiles share the drains out (a scan of
+  // 10,000 rows into 12 groups: 41 us on 3 blocks with 256-row tiles, under 14
+  // on 20 blocks with 32-row ones; from 1.2M rows every warp has a full tile).
+  a.lane_rows = 0;
+  int64_t tile = QM_TILE_ROWS;
+  if (!a.sel && !a.zones && !staged)
+    for (int r = 1; r < QM_R && !a.lane_rows; r *= 2)
+      if (n <= most * warps * 32 * r) {
+        a.lane_rows = r;
+        tile = 32 * r;
+      }
+  const int64_t need = ((n + tile - 1) / tile + warps - 1) / warps;
+  return (int)std::min<int64_t>(most, std::max<int64_t>(need, 1));
 }
 
 // Filter columns to stream through shared memory: every column a term reads,
@@ -1539,6 +1552,33 @@ size_t result_layout(const Plan &pl, qm_outspec &O, int64_t G) {
   return off;
 }
 
+// The finished host buffer's columns and the counters of a result of G rows.
+void fill_result(qm_result *R, const GroupTable &gt, const qm_outspec &O, int64_t G) {
+  const Plan &pl = gt.pl;
+  R->n_rows = G;
+  const uint8_t *h = (const uint8_t *)R->buf.p;
+  for (int k = 0; k < O.n_out; k++) {
+    qm_result::Col c;
+    c.name = pl.meta[k].name;
+    c.dtype = O.o[k].dtype;
+    c.is_key = pl.meta[k].is_key;
+    c.bytes = (size_t)G * dtype_size(c.dtype);
+    c.data = h + O.o[k].offset;
+    if (O.o[k].null_offset >= 0) {
+      c.nulls = h + O.o[k].null_offset;
+      const size_t nb = (size_t)((G + 7) / 8);
+      for (size_t b = 0; b < nb && !c.has_nulls; b++) c.has_nulls = c.nulls[b] != 0;
+    }
+    R->cols.push_back(std::move(c));
+  }
+  R->stats.groups = G;
+  R->stats.strategy = gt.ex.strategy;
+  R->stats.table_capacity = ilog2_ceil(std::max<int64_t>(gt.ex.n_slots, 1));
+  R->stats.retries = gt.retries;
+  R->stats.rows_selected = (int64_t)gt.selected;
+  R->stats.scan_ms = gt.scan_ms;
+}
+
 // ORDER BY / LIMIT / OFFSET over the G emitted rows in ctx->out (layout O):
 // the selected rows in output order into ctx->out2 (layout O2, *G2 rows).
 int post_aggregate(qm_ctx *ctx, const Plan &pl, const qm_outspec &O, int64_t G, qm_outspec &O2, int64_t *G2,
@@ -1824,37 +1864,98 @@ int finish_table(qm_ctx *ctx, GroupTable &gt, qm_result **out, float scan_ms_so_
     G = (int64_t)*(uint64_t *)((char *)ctx->hstatus.p + 32);
   }
 
-  R->n_rows = G;
-  const uint8_t *h = (const uint8_t *)R->buf.p;
-  for (int k = 0; k < O.n_out; k++) {
-    qm_result::Col c;
-    c.name = pl.meta[k].name;
-    c.dtype = O.o[k].dtype;
-    c.is_key = pl.meta[k].is_key;
-    c.bytes = (size_t)G * dtype_size(c.dtype);
-    c.data = h + O.o[k].offset;
-    if (O.o[k].null_offset >= 0) {
-      c.nulls = h + O.o[k].null_offset;
-      const size_t nb = (size_t)((G + 7) / 8);
-      for (size_t b = 0; b < nb && !c.has_nulls; b++) c.has_nulls = c.nulls[b] != 0;
-    }
-    R->cols.push_back(std::move(c));
-  }
-  R->stats.groups = G;
-  R->stats.strategy = ex.strategy;
-  R->stats.table_capacity = ilog2_ceil(std::max<int64_t>(ex.n_slots, 1));
-  R->stats.retries = gt.retries;
-  R->stats.rows_selected = (int64_t)gt.selected;
+  fill_result(R, gt, O, G);
   R->stats.device_ms = (double)(scan_ms_so_far > tail_ms ? scan_ms_so_far : tail_ms);
-  R->stats.scan_ms = gt.scan_ms;
   R->stats.launches = ctx->launches;
   *out = R;
   return QM_OK;
 }
 
+// Queries whose result one block finishes (qm_tail): one
+// scan over a registered table, no post-aggregate clause, and few enough slots
+// for one block to sort.  A hash table has at least 1,024 slots, at most half
+// of them in use; a dense one may fill.
+bool tail_query(const qm_ctx *ctx, const GroupTable &gt, int64_t n_rows) {
+  const Plan &pl = gt.pl;
+  if (pl.post || n_rows <= 0 || ctx->tuning.stage_depth > 0 || ctx->tuning.partitioned > 0) return false;
+  if (pl.key.mode == QK_NONE) return true;
+  if (pl.agg.acc_first < 0) return false;
+  return gt.ex.total_slots <= (pl.key.mode == QK_DIRECT ? QM_TAIL_GROUPS : QM_TAIL_SLOTS);
+}
+
+int scan_args(qm_ctx *ctx, GroupTable &gt, int64_t n, const uint32_t *sel, int bps_cap, qm_scan_args &a, size_t &smem,
+              int &blocks);
+
+// Three launches and one synchronise: the table cleared, the scan, the result
+// written.  *done is false when the general finish has to follow (too many groups for the
+// tail) or st holds an error.
+int run_tail_query(qm_ctx *ctx, GroupTable &gt, int64_t n_rows, qm_result **out, qm_status *st, bool *done) {
+  const Plan &pl = gt.pl;
+  const Exec &ex = gt.ex;
+  *done = false;
+  qm_tail src;
+  memset(&src, 0, sizeof src);
+  src.O = pl.outs;
+  src.rows = pl.key.mode == QK_NONE ? 1 : std::min<int64_t>(ex.total_slots, QM_TAIL_GROUPS);
+  const size_t bytes = result_layout(pl, src.O, src.rows);
+  int rc;
+  if ((rc = ensure(ctx, ctx->tail, 64 + (size_t)src.rows * QM_MAX_OUT)) ||
+      (rc = ensure_host(ctx, ctx->hstatus, sizeof(qm_tail_host))))
+    return rc;
+  qm_result *R = new qm_result();
+  R->pool = ctx->pool;
+  if (!ctx->pool->acquire(bytes + 16, R->buf)) {
+    delete R;
+    return set_err(ctx, QM_ERR_OOM, "pinned result buffer (%zu bytes)", bytes + 16);
+  }
+  src.out = (unsigned char *)R->buf.p;
+  src.host = (qm_tail_host *)ctx->hstatus.p;
+  src.times = (uint64_t *)ctx->tail.p;
+  src.nullbytes = (unsigned char *)ctx->tail.p + 64;
+  src.table = gt.table;
+  src.n_slots = ex.n_slots;
+  src.stride = ex.stride;
+  src.w_count = pl.agg.w_count;
+  src.w_first = pl.agg.w_first;
+  src.status = (qm_status *)ctx->status.p;
+  src.key = pl.key;
+  qm_scan_args a;
+  size_t smem = 0;
+  int blocks = 1;
+  rc = scan_args(ctx, gt, n_rows, nullptr, 0, a, smem, blocks);
+  a.early = 1;
+  cudaError_t e = cudaSuccess;
+  if (!rc) {
+    e = qm_launch_tail_init(gt.table, ex.total_slots, ex.stride, pl.key.mode == QK_HASH, pl.agg, src.status, src.times,
+                            ctx->stream);
+    if (e == cudaSuccess) e = qm_launch_scan(a, blocks, smem, ctx->stream);
+    if (e == cudaSuccess) e = qm_launch_tail_finish(src, ctx->stream);
+    ctx->launches += 3;
+    const cudaError_t se = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = se;
+  }
+  const qm_tail_host *h = src.host;
+  if (!rc && e == cudaSuccess) gt.scan_ms += (double)h->scan_ns * 1e-6;
+  if (rc || e != cudaSuccess || !h->done) {
+    delete R;
+    if (rc) return rc;
+    if (e != cudaSuccess) return set_err(ctx, QM_ERR_CUDA, "small query: %s", cudaGetErrorString(e));
+    *st = h->status;
+    return QM_OK;
+  }
+  *st = h->status;
+  gt.selected = h->status.rows_selected;
+  fill_result(R, gt, src.O, h->groups);
+  R->stats.device_ms = (double)h->device_ns * 1e-6;
+  R->stats.launches = ctx->launches;
+  *out = R;
+  *done = true;
+  return QM_OK;
+}
+
 // Sizes the table for `est_groups` groups and allocates it (from ctx for a
 // one-shot run, owned for a stream).
-int setup_table(qm_ctx *ctx, GroupTable &gt, int64_t est_groups, int64_t direct_size, bool owned) {
+int setup_table(qm_ctx *ctx, GroupTable &gt, int64_t est_groups, int64_t direct_size, bool owned, bool clear = true) {
   Plan &pl = gt.pl;
   Exec &ex = gt.ex;
   if (pl.key.mode == QK_NONE) {
@@ -1874,11 +1975,12 @@ int setup_table(qm_ctx *ctx, GroupTable &gt, int64_t est_groups, int64_t direct_
   int rc = ensure(ctx, buf, bytes);
   if (rc) return rc;
   gt.table = (uint64_t *)buf.p;
-  return init_table(ctx, gt);
+  return clear ? init_table(ctx, gt) : QM_OK;
 }
 
-int run_scan(qm_ctx *ctx, GroupTable &gt, int64_t n, const uint32_t *sel, bool timed = true, int bps_cap = 0) {
-  qm_scan_args a;
+// The arguments and launch shape of a scan of n elements.
+int scan_args(qm_ctx *ctx, GroupTable &gt, int64_t n, const uint32_t *sel, int bps_cap, qm_scan_args &a, size_t &smem,
+              int &blocks) {
   fill_args(gt, a, (qm_status *)ctx->status.p);
   a.n = n;
   a.sel = sel;
@@ -1891,7 +1993,7 @@ int run_scan(qm_ctx *ctx, GroupTable &gt, int64_t n, const uint32_t *sel, bool t
   // per-warp copies pay for their set-up and fold only when every warp has
   // many tiles to aggregate
   if (a.priv && n < PRIV_MIN_ROWS) a.priv = 0;
-  size_t smem = qm_scan_smem_bytes(gt.ex.local_slots, gt.ex.local_hash, gt.pl.agg.n_words, 0, 0, a.priv);
+  smem = qm_scan_smem_bytes(gt.ex.local_slots, gt.ex.local_hash, gt.pl.agg.n_words, 0, 0, a.priv);
   if (!sel && !gt.zones && depth >= 2 && n >= (int64_t)QM_TILE_ROWS * 256) {
     for (; depth >= 2 && !staged; depth--) {
       if (!setup_staging(a.pred, a.stage, depth)) break;
@@ -1904,7 +2006,16 @@ int run_scan(qm_ctx *ctx, GroupTable &gt, int64_t n, const uint32_t *sel, bool t
     }
   }
   if (!staged) memset(&a.stage, 0, sizeof a.stage);
-  int blocks = scan_blocks(ctx, smem, n, staged, bps_cap);
+  blocks = scan_shape(ctx, a, smem, staged, bps_cap);
+  return QM_OK;
+}
+
+int run_scan(qm_ctx *ctx, GroupTable &gt, int64_t n, const uint32_t *sel, bool timed = true, int bps_cap = 0) {
+  qm_scan_args a;
+  size_t smem = 0;
+  int blocks = 1;
+  int rc = scan_args(ctx, gt, n, sel, bps_cap, a, smem, blocks);
+  if (rc) return rc;
   if (timed) CK(cudaEventRecord(ctx->evs0, ctx->stream));
   CK(qm_launch_scan(a, blocks, smem, ctx->stream));
   if (timed) CK(cudaEventRecord(ctx->evs1, ctx->stream));
@@ -2393,7 +2504,7 @@ int qm_ctx_destroy(qm_ctx *ctx) {
                     &ctx->sort_temp, &ctx->counter, &ctx->out, &ctx->hll, &ctx->masks, &ctx->counts,
                     &ctx->offsets, &ctx->sel_out, &ctx->sel_in, &ctx->agg_spare, &ctx->fbits, &ctx->fcounts,
                     &ctx->franks, &ctx->post_last, &ctx->post_hi, &ctx->post_lo, &ctx->post_idx,
-                    &ctx->post_idx2, &ctx->post_k1, &ctx->post_k2, &ctx->post_l1, &ctx->post_l2,
+                    &ctx->tail, &ctx->post_idx2, &ctx->post_k1, &ctx->post_k2, &ctx->post_l1, &ctx->post_l2,
                     &ctx->post_temp, &ctx->out2, &ctx->zstat, &ctx->zones, &ctx->ustat, &ctx->perm,
                     &ctx->wbounds, &ctx->part_counts, &ctx->part_offsets, &ctx->part_bases, &ctx->part_records};
   for (DevBuf *b : bufs) release(*b);
@@ -2675,61 +2786,79 @@ int qm_query_run(qm_ctx *ctx, const qm_table *table, const qm_query *q, qm_resul
   int64_t groups = -1;
   for (int attempt = 0;; attempt++) {
     gt.rows_done = 0;  // every attempt scans the table from its first row
-    CK(cudaMemsetAsync(ctx->status.p, 0, sizeof(qm_status), ctx->stream));
-    CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    if ((rc = setup_table(ctx, gt, est, direct_size, false))) return rc;
-    PartPlan pp;
-    if ((rc = plan_partitioned(ctx, t, gt, est, pp))) return rc;
-    if (pp.on && attempt > 0) pp.spec.rec_cap = t->n_rows;  // a re-run after an overflow: room for every row
-    const int passes = pp.on ? 1 : key_range_passes(gt, t->n_rows, gt.sel_bound);
-    if (pp.on) {
-      if ((rc = run_partitioned(ctx, gt, t->n_rows, pp))) return rc;
-      gt.ex.strategy = 3;
-    } else if (passes <= 1) {
-      if ((rc = run_scan(ctx, gt, t->n_rows, nullptr))) return rc;
-    } else {
-      const qm_pred base = pl.pred;
-      const int64_t span = (gt.ex.n_slots + passes - 1) / passes;
-      CK(cudaEventRecord(ctx->evs0, ctx->stream));
-      for (int p = 0; p < passes; p++) {
-        const int64_t lo = pl.key.base + p * span;
-        const int64_t hi = std::min<int64_t>(pl.key.base + gt.ex.n_slots - 1, lo + span - 1);
-        pl.pred = with_key_range(base, pl.key, lo, hi, p == 0);
-        // one block per SM: fewer warps in flight keep more of the pass's
-        // slots in L2 (200M rows x 16.7M groups: 9.87 -> 9.35 ms)
-        rc = run_scan(ctx, gt, t->n_rows, nullptr, false, KEY_RANGE_BLOCKS_PER_SM);
-        pl.pred = base;
-        if (rc) return rc;
-      }
-      CK(cudaEventRecord(ctx->evs1, ctx->stream));
-      gt.scan_pending = true;
-    }
-    // rank the groups before reading the status: one synchronize for both
-    // (an overflowed table's ranking is discarded with it)
-    gt.rows_done = t->n_rows;
-    const bool ranked = ranked_finish(gt);
-    if (ranked && (rc = launch_rank(ctx, gt))) return rc;
     qm_status st;
-    qm_outspec Ocap = pl.outs;
-    // a dense direct-indexed table (its groups fill most slots) costs no more
-    // to copy laid out for every slot than for its groups
-    const bool dense = pl.key.mode == QK_DIRECT && est * 4 >= gt.ex.total_slots * 3;
-    if (ranked && !pl.post && (dense || result_layout(pl, Ocap, gt.ex.total_slots) <= SPEC_RESULT_BYTES)) {
-      // small or dense result: emitted and copied with the status, one synchronise
-      CK(cudaMemcpyAsync(ctx->hstatus.p, ctx->status.p, sizeof(qm_status), cudaMemcpyDeviceToHost, ctx->stream));
-      if ((rc = finish_table(ctx, gt, out, 0.f, -1, &st, true))) return rc;
-      if (*out) {
+    if ((rc = setup_table(ctx, gt, est, direct_size, false, false))) return rc;
+    const bool tail = tail_query(ctx, gt, t->n_rows);
+    if (tail) {
+      bool done = false;
+      if ((rc = run_tail_query(ctx, gt, t->n_rows, out, &st, &done))) return rc;
+      if (done) {
         (*out)->stats.rows_scanned = t->n_rows;
         (*out)->stats.bytes_scanned = pl.bytes_per_row * t->n_rows;
         return QM_OK;
       }
-    } else {
-      if ((rc = read_status(ctx, &st))) return rc;
-      take_scan_time(ctx, gt, st.error == QM_DEV_OK);
-      if (st.error == QM_DEV_OK) {
+      if (st.error == QM_DEV_OK) {  // more groups than the tail sorts
         gt.selected = st.rows_selected;
-        if (ranked) groups = (int64_t)*(uint64_t *)((char *)ctx->hstatus.p + 32);
+        CK(cudaEventRecord(ctx->ev0, ctx->stream));
         break;
+      }
+    }
+    if (!tail) {
+      PartPlan pp;
+      CK(cudaMemsetAsync(ctx->status.p, 0, sizeof(qm_status), ctx->stream));
+      CK(cudaEventRecord(ctx->ev0, ctx->stream));
+      if ((rc = init_table(ctx, gt))) return rc;
+      if ((rc = plan_partitioned(ctx, t, gt, est, pp))) return rc;
+      if (pp.on && attempt > 0) pp.spec.rec_cap = t->n_rows;  // a re-run after an overflow: room for every row
+      const int passes = pp.on ? 1 : key_range_passes(gt, t->n_rows, gt.sel_bound);
+      if (pp.on) {
+        if ((rc = run_partitioned(ctx, gt, t->n_rows, pp))) return rc;
+        gt.ex.strategy = 3;
+      } else if (passes <= 1) {
+        if ((rc = run_scan(ctx, gt, t->n_rows, nullptr))) return rc;
+      } else {
+        const qm_pred base = pl.pred;
+        const int64_t span = (gt.ex.n_slots + passes - 1) / passes;
+        CK(cudaEventRecord(ctx->evs0, ctx->stream));
+        for (int p = 0; p < passes; p++) {
+          const int64_t lo = pl.key.base + p * span;
+          const int64_t hi = std::min<int64_t>(pl.key.base + gt.ex.n_slots - 1, lo + span - 1);
+          pl.pred = with_key_range(base, pl.key, lo, hi, p == 0);
+          // one block per SM: fewer warps in flight keep more of the pass's
+          // slots in L2 (200M rows x 16.7M groups: 9.87 -> 9.35 ms)
+          rc = run_scan(ctx, gt, t->n_rows, nullptr, false, KEY_RANGE_BLOCKS_PER_SM);
+          pl.pred = base;
+          if (rc) return rc;
+        }
+        CK(cudaEventRecord(ctx->evs1, ctx->stream));
+        gt.scan_pending = true;
+      }
+      // rank the groups before reading the status: one synchronize for both
+      // (an overflowed table's ranking is discarded with it)
+      gt.rows_done = t->n_rows;
+      const bool ranked = ranked_finish(gt);
+      if (ranked && (rc = launch_rank(ctx, gt))) return rc;
+      qm_outspec Ocap = pl.outs;
+      // a dense direct-indexed table (its groups fill most slots) costs no more
+      // to copy laid out for every slot than for its groups
+      const bool dense = pl.key.mode == QK_DIRECT && est * 4 >= gt.ex.total_slots * 3;
+      if (ranked && !pl.post && (dense || result_layout(pl, Ocap, gt.ex.total_slots) <= SPEC_RESULT_BYTES)) {
+        // small or dense result: emitted and copied with the status, one synchronise
+        CK(cudaMemcpyAsync(ctx->hstatus.p, ctx->status.p, sizeof(qm_status), cudaMemcpyDeviceToHost, ctx->stream));
+        if ((rc = finish_table(ctx, gt, out, 0.f, -1, &st, true))) return rc;
+        if (*out) {
+          (*out)->stats.rows_scanned = t->n_rows;
+          (*out)->stats.bytes_scanned = pl.bytes_per_row * t->n_rows;
+          return QM_OK;
+        }
+      } else {
+        if ((rc = read_status(ctx, &st))) return rc;
+        take_scan_time(ctx, gt, st.error == QM_DEV_OK);
+        if (st.error == QM_DEV_OK) {
+          gt.selected = st.rows_selected;
+          if (ranked) groups = (int64_t)*(uint64_t *)((char *)ctx->hstatus.p + 32);
+          break;
+        }
       }
     }
     if (attempt >= 4) return set_err(ctx, QM_ERR_CUDA, "group table overflow after %d regrowths", attempt);
@@ -3504,7 +3633,7 @@ extern "C" int qm_query_run_noalloc(qm_ctx *ctx, int64_t n_rows, int32_t n_cols,
     // per-warp copies pay only on large inputs (the rule of run_scan)
     if (a.priv && n_rows < PRIV_MIN_ROWS) a.priv = 0;
     const size_t smem = qm_scan_smem_bytes(ex.local_slots, ex.local_hash, pl.agg.n_words, 0, 0, a.priv);
-    const int blocks = scan_blocks(ctx, smem, n_rows, false);
+    const int blocks = scan_shape(ctx, a, smem, false);
     CK(qm_launch_scan(a, blocks, smem, ctx->stream));
   }
   qm_status st;
@@ -3982,7 +4111,7 @@ int batch_layout(qm_batch *b) {
     memset(&L.a.stage, 0, sizeof L.a.stage);
     if (L.a.priv && L.a.n < PRIV_MIN_ROWS) L.a.priv = 0;
     L.smem = qm_scan_smem_bytes(g.ex.local_slots, g.ex.local_hash, g.pl.agg.n_words, 0, 0, L.a.priv);
-    L.blocks = scan_blocks(ctx, L.smem, L.a.n, false);
+    L.blocks = scan_shape(ctx, L.a, L.smem, false);
   }
   const int k = std::min(n, 16);
   while ((int)b->side.size() < k) {

@@ -416,6 +416,44 @@ __device__ __forceinline__ uint32_t eval_pred(const qm_pred &P, const ROWS &row,
   return m;
 }
 
+// One row per lane (act: this lane has one).
+__device__ __forceinline__ bool eval_term_row(const qm_term &t, int64_t r, bool act) {
+  bool pass = t.kind == QT_TRUE;
+  if (act && t.kind > QT_FALSE) {
+    if (t.dtype == QM_I32 || t.dtype == QM_I64) {
+      const int64_t v = ld_int(t.data, t.dtype, r);
+      pass = (v >= t.lo && v <= t.hi) == (t.kind == QT_IRANGE);
+    } else {
+      pass = fterm(t, ld_flt(t.data, t.dtype, r));
+    }
+  }
+  if (act && cell_null(t.nulls, r)) pass = t.null_pass != 0;
+  return act && pass;
+}
+
+__device__ __forceinline__ bool eval_pred_row(const qm_pred &P, int64_t r, bool act) {
+  for (int i = 0; i < P.n_and; ++i) {
+    if (!__any_sync(QM_FULL, act)) return false;
+    act = eval_term_row(P.t[i], r, act);
+  }
+  if (P.n_groups > 0) {
+    bool any = false;
+    int b = P.n_and;
+    for (int g = 0; g < P.n_groups; ++g) {
+      bool mg = act && !any;
+      const int e = P.group_end[g];
+      for (int i = b; i < e; ++i) {
+        if (!__any_sync(QM_FULL, mg)) break;
+        mg = eval_term_row(P.t[i], r, mg);
+      }
+      any = any || mg;
+      b = e;
+    }
+    act = any;
+  }
+  return act;
+}
+
 // ---- group keys -------------------------------------------------------------
 // Key word of one row.  special: 0 ordinary, 1 the key equals the empty-slot
 // sentinel (hash mode), 2 NULL key.

@@ -32,6 +32,11 @@ cudaError_t qm_scan_configure(size_t smem_bytes, bool staged, int *blocks_per_sm
 cudaError_t qm_launch_scan(const qm_scan_args &a, int blocks, size_t smem_bytes, cudaStream_t st);
 cudaError_t qm_launch_init_table(uint64_t *t, int64_t n_slots_total, int stride, int hash_keys,
                                  const qm_aggspec &A, int sm_count, cudaStream_t st);
+// Clears a small table and its status ahead of a scan, and the end of such a
+// query (see qm_tail).
+cudaError_t qm_launch_tail_init(uint64_t *t, int64_t n_slots_total, int stride, int hash_keys, const qm_aggspec &A,
+                                qm_status *status, uint64_t *times, cudaStream_t st);
+cudaError_t qm_launch_tail_finish(const qm_tail &T, cudaStream_t st);
 cudaError_t qm_launch_compact(const uint64_t *t, int64_t n_slots_total, int stride, int count_word,
                               int first_word, uint64_t *keys_out, uint32_t *slots_out,
                               unsigned long long *counter, int sm_count, cudaStream_t st);

@@ -245,6 +245,39 @@ struct qm_staging {
   int32_t off[QM_MAX_STAGED];      // byte offset of the column inside a tile buffer
 };
 
+// ---- small results ---------------------------------------------------------------
+// A group table of at most QM_TAIL_SLOTS slots is finished by one block
+// (qm_tail_finish): it sorts the groups by first row and writes the result
+// straight into page-locked host memory, where the general path launches a
+// ranking, an emit and three copies.
+#define QM_TAIL_SLOTS 2050   // slots of the table
+#define QM_TAIL_GROUPS 1024  // groups sorted in shared memory
+struct qm_tail_host {        // page-locked host memory
+  qm_status status;
+  int64_t groups;
+  int32_t done;              // 1: the result is in place; 0: an error, or too many groups
+  int32_t pad;
+  uint64_t scan_ns, device_ns;
+};
+struct qm_tail {
+  unsigned char *out;        // result buffer in host memory (qm_outspec's offsets)
+  qm_tail_host *host;
+  unsigned char *nullbytes;  // device scratch: a byte per nullable output and row
+  uint64_t *times;           // global timer when the clearing launch began and ended
+  int64_t rows;              // rows the result buffer is laid out for
+  const uint64_t *table;     // the group table and its plan, as in qm_scan_args
+  int64_t n_slots;
+  int32_t stride;
+  int32_t w_count, w_first;
+  int32_t pad;
+  qm_status *status;
+  qm_keyspec key;
+  qm_outspec O;
+};
+struct qm_init_words {
+  uint64_t w[QM_MAX_WORDS];
+};
+
 struct qm_scan_args {
   qm_pred pred;
   qm_keyspec key;
@@ -266,6 +299,9 @@ struct qm_scan_args {
   int32_t local_rep;     // log2 of the copies of each direct block-local slot
                          // (lane l updates copy l mod copies; local_slots
                          // counts the copies); 0 for hashed or deduplicated
+  int32_t lane_rows;     // rows a lane takes of a tile: 0 as many as QM_R, else
+                         // tiles of 32 * lane_rows rows (few rows: more warps)
+  int32_t early;         // launched behind qm_tail_init, overlapping its end
   int32_t pad;
   const uint32_t *zones; // zones (QM_ZONE_TILES tiles each) to scan, ascending, or null: every tile
   int64_t n_zone_tiles;  // zones: tiles covered (count of zones x QM_ZONE_TILES)

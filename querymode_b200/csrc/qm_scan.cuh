@@ -83,9 +83,12 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
     for (int d = 0; d < S.depth; ++d) mbar_init(&mbar[d], 1);
     fence_async_shared();
   }
+  // launched early behind the clearing of a small table (no effect otherwise)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();
 
-  const int64_t n_tiles = (a.n + QM_TILE_ROWS - 1) / QM_TILE_ROWS;
+  const int tile_rows = a.lane_rows ? 32 * a.lane_rows : QM_TILE_ROWS;
+  const int64_t n_tiles = (a.n + tile_rows - 1) / tile_rows;
   const int64_t full_tiles = a.n / QM_TILE_ROWS;
   const int64_t gwarps = (int64_t)gridDim.x * warps;
   const int64_t first = (int64_t)blockIdx.x * warps + warp;
@@ -122,7 +125,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   for (int64_t v = first; v < n_virtual; v += gwarps, ++k) {
     const int64_t tile = tile_of(v);
     if (tile >= n_tiles) continue;  // the table's last zone is partial
-    const int64_t e0 = tile * QM_TILE_ROWS;
+    const int64_t e0 = tile * tile_rows;
     uint32_t m = 0;
     if (STAGED && tile < full_tiles) {
       __syncwarp();
@@ -145,6 +148,17 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       const int tot = (int)base - qn;
       qn = (int)base;
       selected += tot;
+    } else if (!SEL && a.lane_rows) {
+      // few rows: short tiles, a row of the warp's 32 per lane and step, so
+      // that the serial drains of a tile spread over the idle warps
+      for (int j = 0; j < a.lane_rows; ++j) {
+        const int64_t row = e0 + j * 32 + lane;
+        const bool pass = eval_pred_row(a.pred, row, row < a.n);
+        const uint32_t bal = __ballot_sync(QM_FULL, pass);
+        if (pass) queue[qn + __popc(bal & lt)] = (uint32_t)row;
+        qn += __popc(bal);
+        selected += __popc(bal);
+      }
     } else if (!SEL && a.vec_ok && e0 + QM_TILE_ROWS <= a.n) {
       // full dense tile: the lane's rows are r0 .. r0+7
       const int64_t r0 = e0 + (int64_t)lane * QM_R;
@@ -238,6 +252,23 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
     }
     merge_block(a, lkeys, lw);
   }
+}
+
+// Launch of one instantiation: `early`, overlapping the end of the clearing
+// launch ahead of it (the kernel waits for it before it touches the table).
+template <class KERNEL>
+inline cudaError_t launch_scan_kernel(KERNEL kernel, const qm_scan_args &a, int blocks, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)blocks);
+  c.blockDim = dim3(QM_SCAN_THREADS);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = a.early ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, a);
 }
 
 }  // namespace qm

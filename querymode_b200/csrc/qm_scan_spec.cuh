@@ -45,8 +45,7 @@ cudaError_t QM_SPEC_FN(_launch)(const qm_scan_args &a, int dd, int kk, int ft, i
   using namespace qm;
 #define QM_LAUNCH_(DD, KK, FT, LM)                                                                              \
   if (dd == DD && (kk == KK || KK == QM_KK_ANY) && ft >= FT && (lm == LM || LM == QM_LM_ANY)) {                 \
-    qm_scan_kernel<false, false, DD, QM_SPEC_NV, KK, FT, LM><<<blocks, QM_SCAN_THREADS, smem, st>>>(a);         \
-    return cudaGetLastError();                                                                                  \
+    return launch_scan_kernel(qm_scan_kernel<false, false, DD, QM_SPEC_NV, KK, FT, LM>, a, blocks, smem, st);    \
   }
   QM_SPEC_LIST(QM_LAUNCH_)
 #undef QM_LAUNCH_
