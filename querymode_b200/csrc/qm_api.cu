@@ -982,6 +982,41 @@ int build_agg(qm_ctx *ctx, const qm_query *q, const ColEnv &env, Plan &pl, std::
     }
     pl.meta.push_back({name, o.dtype, 0, ag.fn != QM_AGG_COUNT});
   }
+  // FIRST and the first MIN / MAX come first: a probe of a hash slot reads
+  // them with the key (slot_head)
+  {
+    std::vector<int> order;
+    auto is_head = [&](int kind) {
+      return kind == QA_FIRST || kind == QA_IMIN || kind == QA_IMAX || kind == QA_FMIN || kind == QA_FMAX;
+    };
+    for (int i = 0; i < A.n_accs; i++)
+      if (is_head(A.acc[i].kind)) order.push_back(i);
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int x, int y) { return (A.acc[x].kind == QA_FIRST) > (A.acc[y].kind == QA_FIRST); });
+    for (int i = 0; i < A.n_accs; i++)
+      if (!is_head(A.acc[i].kind)) order.push_back(i);
+    int to[QM_MAX_WORDS] = {0}, at = 0;
+    uint64_t init[QM_MAX_WORDS] = {0};
+    for (int i : order) {
+      qm_acc &ac = A.acc[i];
+      const int width = (ac.kind == QA_ISUM || ac.kind == QA_FSUM) ? 2 : 1;
+      for (int w = 0; w < width; w++) {
+        to[ac.word + w] = at + w;
+        init[at + w] = A.init[ac.word + w];
+      }
+      ac.word = at;
+      at += width;
+    }
+    memcpy(A.init, init, sizeof init);
+    for (int k = 0; k < O.n_out; k++) {
+      qm_out &o = O.o[k];
+      if (o.kind == QO_KEY) continue;
+      o.word = to[o.word];
+      o.nn_word = to[o.nn_word];
+      if (o.zero_word >= 0) o.zero_word = to[o.zero_word];
+      if (o.fixed) o.nf_word = to[o.nf_word];
+    }
+  }
   A.n_vcols = (int)vcols.size();
   A.w_count = A.acc[A.acc_count].word;
   A.w_first = A.acc_first >= 0 ? A.acc[A.acc_first].word : -1;
@@ -1012,7 +1047,6 @@ int build_agg(qm_ctx *ctx, const qm_query *q, const ColEnv &env, Plan &pl, std::
 // ------------------------------------------------------------ execution
 struct Exec {
   int64_t n_slots = 1;  // QK_DIRECT size / QK_HASH capacity
-  int log2cap = 0;
   int64_t total_slots = 1;
   int stride = 1;
   int local_slots = 0;
@@ -1029,6 +1063,14 @@ int ilog2_ceil(int64_t x) {
   int l = 0;
   while (((int64_t)1 << l) < x) l++;
   return l;
+}
+
+// Slots of a hash table for an estimated number of groups: 2.1 each, any
+// number.  At 1.6 the longest of a warp's 32 probes grows (20M rows into
+// 500,000 groups: scan 0.76 -> 0.94 ms); rounded up to a power of two (2.1-4.3
+// each) the table is larger to clear, rank and emit and no faster to scan.
+int64_t hash_slots(int64_t groups) {
+  return std::min<int64_t>((int64_t)1 << 31, std::max<int64_t>(1024, groups * 2 + groups / 8));
 }
 
 constexpr size_t LOCAL_BUDGET = 40 * 1024;  // bytes of the block-local hash table
@@ -1053,9 +1095,12 @@ int local_copies(int64_t slots, int64_t per_slot) {
   return r;
 }
 
-void choose_layout(const Plan &pl, int64_t est_groups, Exec &ex, const qm_tuning &tu) {
+// align: hash slots may be padded to 32 bytes (tables of the library's own;
+// not partial rows, whose words the slots are, nor the fixed scratch array).
+void choose_layout(const Plan &pl, int64_t est_groups, Exec &ex, const qm_tuning &tu, bool align) {
   const int words = pl.agg.n_words;
   ex.stride = 1 + words;
+  if (align && pl.key.mode == QK_HASH && ((words + 4) & ~3) - 1 <= QM_MAX_WORDS) ex.stride = (words + 4) & ~3;
   ex.total_slots = ex.n_slots + special_slots(pl.key.mode);
   const int64_t per_slot = (int64_t)words * 8;
   ex.priv = 0;
@@ -1090,7 +1135,8 @@ void choose_layout(const Plan &pl, int64_t est_groups, Exec &ex, const qm_tuning
       while ((int64_t)(L * 2) * (per_slot + 8) <= (int64_t)LOCAL_WIDE_BUDGET) L *= 2;
     if (tu.local_slots > 0) {
       L = tu.local_slots;
-      while (L > 1 && (int64_t)L * (per_slot + 8) > (int64_t)200 * 1024) L /= 2;  // fit shared memory
+      while (L > 4 && (int64_t)L * (per_slot + 8) > (int64_t)200 * 1024) L /= 2;  // fit shared memory
+      L = std::max(L, 4);  // slots are looked up in buckets of four
     }
     ex.local_slots = L;
     ex.local_hash = 1;
@@ -1107,8 +1153,8 @@ void choose_layout(const Plan &pl, int64_t est_groups, Exec &ex, const qm_tuning
 std::mutex g_cfg_mu;
 // Occupancy answers are fixed per (device, kernel, shared memory) and the
 // runtime queries cost tens of microseconds under g_cfg_mu, which every
-// planning thread takes: they are cached.  Kernel ids: -1 / -2 the generic
-// scan (direct / staged), >= 0 a batched class.
+// planning thread takes: they are cached.  Kernel ids: below 0 a scan
+// (-1 - qm_scan_kernel_id), else a batched class.
 std::map<std::tuple<int, int, size_t>, int> g_occ;
 // The largest dynamic shared-memory limit set on each batched class kernel:
 // the limit is only ever raised, so a lane never lowers it under another
@@ -1122,11 +1168,11 @@ int scan_shape(qm_ctx *ctx, qm_scan_args &a, size_t smem, bool staged, int cap =
   int bps = 1;
   {
     std::lock_guard<std::mutex> lk(g_cfg_mu);
-    const auto key = std::make_tuple(ctx->device, staged ? -2 : -1, smem);
+    const auto key = std::make_tuple(ctx->device, -1 - qm_scan_kernel_id(a), smem);
     auto it = g_occ.find(key);
     if (it != g_occ.end()) {
       bps = it->second;
-    } else if (qm_scan_configure(smem, staged, &bps) != cudaSuccess) {
+    } else if (qm_scan_occupancy(a, smem, &bps) != cudaSuccess) {
       cudaGetLastError();
       bps = 1;
     } else {
@@ -1140,18 +1186,20 @@ int scan_shape(qm_ctx *ctx, qm_scan_args &a, size_t smem, bool staged, int cap =
     bps = cap;
   }
   const int64_t warps = QM_SCAN_THREADS / 32, most = (int64_t)ctx->sm_count * bps;
-  // A tile of 256 rows is drained 32 rows at a time, one after another: while
+  // A warp's 512 rows are drained 32 at a time, one after another: while
   // warps would stay idle, shorter tiles share the drains out (a scan of
-  // 10,000 rows into 12 groups: 41 us on 3 blocks with 256-row tiles, under 14
-  // on 20 blocks with 32-row ones; from 1.2M rows every warp has a full tile).
+  // 10,000 rows into 12 groups: 41 us on 3 blocks with 256 rows a warp, under 14
+  // on 20 blocks with 32).  Single tiles of 256 rows until every warp has four
+  // pairs: fewer pairs leave the last round of them half empty (5M rows, 2.1
+  // pairs a warp: totals 145 us with pairs, 127 with single tiles).
   a.lane_rows = 0;
-  int64_t tile = QM_TILE_ROWS;
-  if (!a.sel && !a.zones && !staged)
+  int64_t tile = staged ? QM_TILE_ROWS : QM_SCAN_ROWS;
+  if (!a.sel && !a.zones && !staged) {
     for (int r = 1; r < QM_R && !a.lane_rows; r *= 2)
-      if (n <= most * warps * 32 * r) {
-        a.lane_rows = r;
-        tile = 32 * r;
-      }
+      if (n <= most * warps * 32 * r) a.lane_rows = r;
+    if (!a.lane_rows && n <= most * warps * QM_SCAN_ROWS * 4) a.lane_rows = QM_R;
+    if (a.lane_rows) tile = 32 * a.lane_rows;
+  }
   const int64_t need = ((n + tile - 1) / tile + warps - 1) / warps;
   return (int)std::min<int64_t>(most, std::max<int64_t>(need, 1));
 }
@@ -1473,7 +1521,7 @@ void fill_args(const GroupTable &gt, qm_scan_args &a, qm_status *st) {
   a.table = gt.table;
   a.n_slots = gt.ex.n_slots;
   a.stride = gt.ex.stride;
-  a.log2cap = gt.ex.log2cap;
+  a.head = gt.pl.key.mode == QK_HASH && gt.ex.stride % 4 == 0 && ((uintptr_t)gt.table & 31) == 0;
   a.local_slots = gt.ex.local_slots;
   a.local_hash = gt.ex.local_hash;
   a.dedupe = gt.ex.dedupe;
@@ -1873,8 +1921,7 @@ int finish_table(qm_ctx *ctx, GroupTable &gt, qm_result **out, float scan_ms_so_
 
 // Queries whose result one block finishes (qm_tail): one
 // scan over a registered table, no post-aggregate clause, and few enough slots
-// for one block to sort.  A hash table has at least 1,024 slots, at most half
-// of them in use; a dense one may fill.
+// for one block to sort.  (A dense table may fill.)
 bool tail_query(const qm_ctx *ctx, const GroupTable &gt, int64_t n_rows) {
   const Plan &pl = gt.pl;
   if (pl.post || n_rows <= 0 || ctx->tuning.stage_depth > 0 || ctx->tuning.partitioned > 0) return false;
@@ -1963,12 +2010,11 @@ int setup_table(qm_ctx *ctx, GroupTable &gt, int64_t est_groups, int64_t direct_
   } else if (pl.key.mode == QK_DIRECT) {
     ex.n_slots = direct_size;
   } else {
-    int64_t want = std::max<int64_t>(1024, est_groups * 2 + est_groups / 8);
-    ex.log2cap = ilog2_ceil(want);
-    if (ex.log2cap > 31) ex.log2cap = 31;
-    ex.n_slots = (int64_t)1 << ex.log2cap;
+    // a stream's table has room for the next batches' groups: a power of two,
+    // as grow_table makes it
+    ex.n_slots = owned ? (int64_t)1 << std::min(31, ilog2_ceil(hash_slots(est_groups))) : hash_slots(est_groups);
   }
-  choose_layout(pl, est_groups, ex, ctx->tuning);
+  choose_layout(pl, est_groups, ex, ctx->tuning, !owned);
   size_t bytes = (size_t)ex.total_slots * ex.stride * 8;
   DevBuf &buf = owned ? gt.own : ctx->table;
   if (owned && !buf.p && ctx->agg_spare.bytes >= bytes) std::swap(buf, ctx->agg_spare);
@@ -2962,11 +3008,12 @@ int stage_selection(qm_ctx *ctx, const uint32_t *sel, int64_t n_sel, const uint3
 // Grow a streaming hash table so that `upper` groups keep the load <= ~0.5.
 int grow_table(qm_ctx *ctx, GroupTable &gt, int64_t upper) {
   Exec &ex = gt.ex;
-  if (gt.pl.key.mode != QK_HASH || upper * 2 + upper / 8 <= ex.n_slots) return QM_OK;
+  if (gt.pl.key.mode != QK_HASH || hash_slots(upper) <= ex.n_slots) return QM_OK;
   Exec nx = ex;
-  nx.log2cap = ilog2_ceil(std::max<int64_t>(1024, upper * 2 + upper / 8));
-  if (nx.log2cap > 31) return set_err(ctx, QM_ERR_OOM, "group table would exceed 2^31 slots");
-  nx.n_slots = (int64_t)1 << nx.log2cap;
+  // (a power of two: growing push by push re-hashes rarely)
+  const int log2cap = ilog2_ceil(hash_slots(upper));
+  if (log2cap > 31) return set_err(ctx, QM_ERR_OOM, "group table would exceed 2^31 slots");
+  nx.n_slots = (int64_t)1 << log2cap;
   nx.total_slots = nx.n_slots + 2;
   DevBuf nb;
   int rc = ensure(ctx, nb, (size_t)nx.total_slots * nx.stride * 8);
@@ -2981,7 +3028,7 @@ int grow_table(qm_ctx *ctx, GroupTable &gt, int64_t upper) {
   }
   CK(cudaMemsetAsync(ctx->status.p, 0, sizeof(qm_status), ctx->stream));
   CK(qm_launch_rehash(gt.table, ex.n_slots, ex.stride, gt.pl.agg.acc[gt.pl.agg.acc_count].word, tmp.table,
-                      nx.log2cap, (qm_status *)ctx->status.p, ctx->sm_count, ctx->stream));
+                      nx.n_slots, (qm_status *)ctx->status.p, ctx->sm_count, ctx->stream));
   // the two reserved slots (sentinel-valued key, NULL key) move as they are
   CK(cudaMemcpyAsync(tmp.table + nx.n_slots * nx.stride, gt.table + ex.n_slots * ex.stride,
                      (size_t)2 * ex.stride * 8, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -2998,7 +3045,7 @@ int grow_table(qm_ctx *ctx, GroupTable &gt, int64_t upper) {
   gt.own = nb;
   gt.table = tmp.table;
   // local-table choice may change with the new size
-  choose_layout(gt.pl, upper, nx, ctx->tuning);
+  choose_layout(gt.pl, upper, nx, ctx->tuning, false);
   gt.ex = nx;
   return QM_OK;
 }
@@ -3589,11 +3636,11 @@ extern "C" int qm_query_run_noalloc(qm_ctx *ctx, int64_t n_rows, int32_t n_cols,
   if (pl.key.mode == QK_NONE) {
     ex.n_slots = 1;
   } else {
-    ex.log2cap = ilog2_ceil(std::max<int64_t>(1024, max_groups * 2 + max_groups / 8));
-    if (ex.log2cap > 30) return set_err(ctx, QM_ERR_CAPACITY, "max_groups too large for the scratch array");
-    ex.n_slots = (int64_t)1 << ex.log2cap;
+    const int log2cap = ilog2_ceil(std::max<int64_t>(1024, max_groups * 2 + max_groups / 8));
+    if (log2cap > 30) return set_err(ctx, QM_ERR_CAPACITY, "max_groups too large for the scratch array");
+    ex.n_slots = (int64_t)1 << log2cap;
   }
-  choose_layout(pl, max_groups, ex, ctx->tuning);
+  choose_layout(pl, max_groups, ex, ctx->tuning, false);
   const int64_t G_cap = pl.key.mode == QK_NONE ? 1 : max_groups;
   const size_t status_off = 0;
   const size_t table_off = 256;
@@ -3941,7 +3988,7 @@ int batch_layout(qm_batch *b) {
       }
     }
     table_off[i] = words;
-    words += ex.total_slots * ex.stride;
+    words += (ex.total_slots * ex.stride + 3) & ~(int64_t)3;  // tables start on 32-byte boundaries
   }
   plan_waves(b);
   int rc;
@@ -4383,11 +4430,9 @@ int batch_plan_one(qm_batch *b, int i, const qm_table *table, const qm_query *qu
   } else if (gt.pl.key.mode == QK_DIRECT) {
     ex.n_slots = direct_size;
   } else {
-    int64_t want = std::max<int64_t>(1024, est * 2 + est / 8);
-    ex.log2cap = ilog2_ceil(want);
-    ex.n_slots = (int64_t)1 << ex.log2cap;
+    ex.n_slots = hash_slots(est);
   }
-  choose_layout(gt.pl, est, ex, ctx->tuning);
+  choose_layout(gt.pl, est, ex, ctx->tuning, true);
   b->est[i] = est;
   b->ex_plan[i] = ex;
   qm_bq &qb = b->bq[i];
@@ -4410,7 +4455,7 @@ int64_t batch_query_bytes(const qm_batch *b, int i) {
   const GroupTable &gt = b->gts[i];
   const qm_bq &q = b->bq[i];
   const int64_t total_slots = gt.ex.n_slots + special_slots(gt.pl.key.mode);
-  const int64_t table = total_slots * (1 + gt.pl.agg.n_words) * 8;
+  const int64_t table = total_slots * gt.ex.stride * 8 + 32;
   const int64_t gmax = q.none ? 1 : std::min<int64_t>(total_slots, std::max<int64_t>(b->rows[i], 1));
   int64_t res = 0;
   for (int k = 0; k < q.outs.n_out; k++) res += (gmax * q.width[k] + 15) / 16 * 16 + (q.nullable[k] ? 2 * gmax + 64 : 0);
@@ -4462,7 +4507,7 @@ int qm_batch_set_tuning(qm_batch *b, int32_t chunk_tiles, int32_t local_kb, int3
   if (blocks_per_sm >= 0) b->bps = blocks_per_sm;
   cudaSetDevice(b->ctx->device);
   // rebuild block-local table choices from the planner's, then re-lay out
-  for (int i = 0; i < b->n; i++) choose_layout(b->gts[i].pl, b->est[i], b->gts[i].ex, b->ctx->tuning);
+  for (int i = 0; i < b->n; i++) choose_layout(b->gts[i].pl, b->est[i], b->gts[i].ex, b->ctx->tuning, true);
   return batch_layout(b);
 }
 
@@ -4470,7 +4515,7 @@ int qm_batch_set_waves(qm_batch *b, int32_t waves) {
   if (!b || waves < 0) return QM_ERR_INVALID;
   cudaSetDevice(b->ctx->device);
   b->waves_req = waves;
-  for (int i = 0; i < b->n; i++) choose_layout(b->gts[i].pl, b->est[i], b->gts[i].ex, b->ctx->tuning);
+  for (int i = 0; i < b->n; i++) choose_layout(b->gts[i].pl, b->est[i], b->gts[i].ex, b->ctx->tuning, true);
   return batch_layout(b);
 }
 

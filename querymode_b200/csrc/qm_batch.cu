@@ -78,7 +78,6 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ qm_scan_args P;
   __shared__ int s_chunk;
-  __shared__ int l_used;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int warps = blockDim.x >> 5;
@@ -106,7 +105,6 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       const uint32_t *src = reinterpret_cast<const uint32_t *>(&bq[ch.q].a);
       uint32_t *dst = reinterpret_cast<uint32_t *>(&P);
       for (int i = threadIdx.x; i < (int)(sizeof(qm_scan_args) / 4); i += blockDim.x) dst[i] = __ldg(src + i);
-      if (threadIdx.x == 0) l_used = 0;
       __syncthreads();
       const int L = P.local_slots;
       lw = lkeys + (P.local_hash ? L : 0);
@@ -119,6 +117,10 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       cur = ch.q;
     }
     const int L = P.local_slots;
+    const char *pf_base;
+    int pf_elem;
+    prefetch_column(P.pred, lane, pf_base, pf_elem);
+    uint32_t pf_want = ~0u;
     int qn = 0;
     for (int64_t tile = ch.tile0 + warp; tile < ch.tile1; tile += warps) {
       const int64_t e0 = tile * QM_TILE_ROWS;
@@ -126,8 +128,9 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       const int64_t r0 = e0 + (int64_t)lane * QM_R;
       if (P.vec_ok && e0 + QM_TILE_ROWS <= P.n) {
         const int64_t nxt = tile + warps;
-        if (nxt < ch.tile1 && (nxt + 1) * QM_TILE_ROWS <= P.n) prefetch_tile_l2(P.pred, nxt * QM_TILE_ROWS, lane);
-        m = eval_pred_contig(P.pred, r0, (1u << QM_R) - 1);
+        if (nxt < ch.tile1 && (nxt + 1) * QM_TILE_ROWS <= P.n)
+          prefetch_tile_l2(pf_base, pf_elem, pf_want, nxt * QM_TILE_ROWS, QM_TILE_ROWS, lane);
+        m = eval_pred_contig<1>(P.pred, r0, (1u << QM_R) - 1, pf_want);
       } else {
         int64_t rowv[QM_R];
         m = 0;
@@ -157,14 +160,14 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
         const int64_t row = queue[qn - 32 + lane];
         __syncwarp();
         qn -= 32;
-        drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, &l_used, lane, true, row);
+        drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, lane, true, row);
       }
     }
     if (qn > 0) {
       const bool active = lane < qn;
       const int64_t row = active ? (int64_t)queue[lane] : 0;
       __syncwarp();
-      drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, &l_used, lane, active, row);
+      drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, lane, active, row);
     }
     __syncthreads();
   }

@@ -306,11 +306,11 @@ __global__ void qm_compact_groups(const uint64_t *t, int64_t n_slots_total, int 
 // Move the occupied hash slots of a table into a larger one (keys are
 // unique, so each new slot has one writer and the words are plain copies).
 __global__ void qm_rehash(const uint64_t *old_t, int64_t old_cap, int stride, int count_word, uint64_t *new_t,
-                          int log2cap, qm_status *st) {
+                          int64_t n_slots, qm_status *st) {
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < old_cap; s += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t *src = old_t + s * stride;
     if (src[1 + count_word] == 0) continue;
-    const int64_t ns = global_find(new_t, stride, log2cap, src[0], 1 << 12, st);
+    const int64_t ns = global_find(new_t, stride, n_slots, src[0], 1 << 12, st);
     if (ns < 0) {
       set_error(st, QM_DEV_OVERFLOW);
       continue;
@@ -1661,50 +1661,59 @@ int value_features(const qm_aggspec &A) {
 }
 }  // namespace
 
-cudaError_t qm_scan_configure(size_t smem_bytes, bool staged, int *blocks_per_sm) {
-  if (smem_bytes > (size_t)QM_SCAN_SMEM_MAX) return cudaErrorInvalidValue;
+struct scan_choice {
+  int dd, kk, ft, lm;
+  bool spec;  // one of the kernels specialised for the value-column count
+};
+
+static scan_choice choose_scan(const qm_scan_args &a) {
+  scan_choice c;
+  c.dd = a.dedupe != 0 ? 1 : 0;
+  c.kk = c.dd ? QM_KK_ANY : key_kind(a.key);
+  c.ft = value_features(a.agg);
+  c.lm = c.dd ? QM_LM_ANY
+              : (a.local_slots > 0 && !a.local_hash ? QM_LM_DIRECT : (a.key.mode == QK_HASH && a.head ? QM_LM_HASH : QM_LM_ANY));
+  // fixed-point (deterministic) sums run in the run-time-plan kernels only
+  c.spec = !a.sel && a.stage.n == 0 && a.agg.n_vcols <= QM_SPEC_NV_MAX && c.ft != QM_FT_FULL;
+  return c;
+}
+
+int qm_scan_kernel_id(const qm_scan_args &a) {
+  const scan_choice c = choose_scan(a);
+  if (!c.spec) return (c.dd | (a.sel ? 2 : 0) | (a.stage.n > 0 ? 4 : 0));
+  return 8 + (((a.agg.n_vcols * 4 + c.kk) * 4 + c.ft) * 3 + c.lm) * 2 + c.dd;
+}
+
+static cudaError_t scan_dispatch(const qm_scan_args &a, int blocks, size_t smem, cudaStream_t st, int *per_sm) {
   cudaError_t e = scan_attrs_once();
   if (e != cudaSuccess) return e;
-  if (staged)
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        blocks_per_sm, qm_scan_kernel<false, true, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>, QM_SCAN_THREADS, smem_bytes);
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      blocks_per_sm, qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>, QM_SCAN_THREADS, smem_bytes);
+  const scan_choice c = choose_scan(a);
+  if (c.spec) {
+    switch (a.agg.n_vcols) {
+      case 0: return qm_scan_nv0_launch(a, c.dd, c.kk, c.ft, c.lm, blocks, smem, st, per_sm);
+      case 1: return qm_scan_nv1_launch(a, c.dd, c.kk, c.ft, c.lm, blocks, smem, st, per_sm);
+      case 2: return qm_scan_nv2_launch(a, c.dd, c.kk, c.ft, c.lm, blocks, smem, st, per_sm);
+      case 3: return qm_scan_nv3_launch(a, c.dd, c.kk, c.ft, c.lm, blocks, smem, st, per_sm);
+      case 4: return qm_scan_nv4_launch(a, c.dd, c.kk, c.ft, c.lm, blocks, smem, st, per_sm);
+    }
+  }
+#define QM_GENERIC(SEL, STAGED, DD)                                                                                \
+  launch_scan_kernel(qm_scan_kernel<SEL, STAGED, DD, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>, a, blocks, smem, \
+                     st, per_sm)
+  if (a.sel) return c.dd ? QM_GENERIC(true, false, 1) : QM_GENERIC(true, false, 0);
+  if (a.stage.n > 0) return c.dd ? QM_GENERIC(false, true, 1) : QM_GENERIC(false, true, 0);
+  return c.dd ? QM_GENERIC(false, false, 1) : QM_GENERIC(false, false, 0);
+#undef QM_GENERIC
+}
+
+cudaError_t qm_scan_occupancy(const qm_scan_args &a, size_t smem_bytes, int *blocks_per_sm) {
+  if (smem_bytes > (size_t)QM_SCAN_SMEM_MAX) return cudaErrorInvalidValue;
+  return scan_dispatch(a, 1, smem_bytes, nullptr, blocks_per_sm);
 }
 
 cudaError_t qm_launch_scan(const qm_scan_args &a, int blocks, size_t smem_bytes, cudaStream_t st) {
   if (a.n <= 0) return cudaSuccess;
-  cudaError_t e = scan_attrs_once();
-  if (e != cudaSuccess) return e;
-  const int dd = a.dedupe != 0 ? 1 : 0;
-  if (!a.sel && a.stage.n == 0 && a.agg.n_vcols <= QM_SPEC_NV_MAX) {
-    const int ft = value_features(a.agg);
-    if (ft != QM_FT_FULL) {  // fixed-point (deterministic) sums run in the run-time-plan kernels only
-      const int kk = dd ? QM_KK_ANY : key_kind(a.key);
-      const int lm = !dd && a.local_slots > 0 && !a.local_hash ? QM_LM_DIRECT : QM_LM_ANY;
-      switch (a.agg.n_vcols) {
-        case 0: return qm_scan_nv0_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
-        case 1: return qm_scan_nv1_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
-        case 2: return qm_scan_nv2_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
-        case 3: return qm_scan_nv3_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
-        case 4: return qm_scan_nv4_launch(a, dd, kk, ft, lm, blocks, smem_bytes, st);
-      }
-    }
-  }
-  if (a.sel) {
-    if (dd) qm_scan_kernel<true, false, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
-    else qm_scan_kernel<true, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
-  } else if (a.stage.n > 0) {
-    if (dd) qm_scan_kernel<false, true, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
-    else qm_scan_kernel<false, true, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY><<<blocks, QM_SCAN_THREADS, smem_bytes, st>>>(a);
-  } else if (dd) {
-    return launch_scan_kernel(qm_scan_kernel<false, false, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>, a, blocks,
-                              smem_bytes, st);
-  } else {
-    return launch_scan_kernel(qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>, a, blocks,
-                              smem_bytes, st);
-  }
-  return cudaGetLastError();
+  return scan_dispatch(a, blocks, smem_bytes, st, nullptr);
 }
 
 cudaError_t qm_launch_init_table(uint64_t *t, int64_t n_slots_total, int stride, int hash_keys,
@@ -2054,10 +2063,10 @@ cudaError_t qm_launch_hll(const qm_keyspec &K, int64_t n, uint32_t *regs, int sm
 }
 
 cudaError_t qm_launch_rehash(const uint64_t *old_t, int64_t old_cap, int stride, int count_word, uint64_t *new_t,
-                             int log2cap, qm_status *st, int sm_count, cudaStream_t stream) {
+                             int64_t n_slots, qm_status *st, int sm_count, cudaStream_t stream) {
   if (old_cap <= 0) return cudaSuccess;
   int blocks = (int)std::min<int64_t>((old_cap + 255) / 256, (int64_t)sm_count * 8);
-  qm_rehash<<<blocks, 256, 0, stream>>>(old_t, old_cap, stride, count_word, new_t, log2cap, st);
+  qm_rehash<<<blocks, 256, 0, stream>>>(old_t, old_cap, stride, count_word, new_t, n_slots, st);
   return cudaGetLastError();
 }
 

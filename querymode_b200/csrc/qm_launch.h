@@ -17,8 +17,7 @@
 #define QM_DECL_SPEC(N)                                                                        \
   cudaError_t qm_scan_nv##N##_attr(int max_smem);                                           \
   cudaError_t qm_scan_nv##N##_launch(const qm_scan_args &a, int dd, int kk, int ft, int lm, int blocks, \
-                                     size_t smem, \
-                                     cudaStream_t st);
+                                     size_t smem, cudaStream_t st, int *per_sm);
 QM_DECL_SPEC(0)
 QM_DECL_SPEC(1)
 QM_DECL_SPEC(2)
@@ -28,7 +27,10 @@ QM_DECL_SPEC(4)
 
 size_t qm_scan_smem_bytes(int local_slots, int local_hash, int n_words, int stage_tile_bytes, int stage_depth,
                           int priv);
-cudaError_t qm_scan_configure(size_t smem_bytes, bool staged, int *blocks_per_sm);
+// Blocks per SM of the kernel that the plan's launch takes, and a number that
+// is the same for launches of one kernel.
+cudaError_t qm_scan_occupancy(const qm_scan_args &a, size_t smem_bytes, int *blocks_per_sm);
+int qm_scan_kernel_id(const qm_scan_args &a);
 cudaError_t qm_launch_scan(const qm_scan_args &a, int blocks, size_t smem_bytes, cudaStream_t st);
 cudaError_t qm_launch_init_table(uint64_t *t, int64_t n_slots_total, int stride, int hash_keys,
                                  const qm_aggspec &A, int sm_count, cudaStream_t st);
@@ -130,7 +132,7 @@ cudaError_t qm_launch_sample_pred(const qm_pred &P, int64_t n, int n_samples, un
                                   cudaStream_t st);
 cudaError_t qm_launch_hll(const qm_keyspec &K, int64_t n, uint32_t *regs, int sm_count, cudaStream_t st);
 cudaError_t qm_launch_rehash(const uint64_t *old_t, int64_t old_cap, int stride, int count_word, uint64_t *new_t,
-                             int log2cap, qm_status *st, int sm_count, cudaStream_t stream);
+                             int64_t n_slots, qm_status *st, int sm_count, cudaStream_t stream);
 cudaError_t qm_launch_check_selection(const uint32_t *sel, int64_t n_sel, int64_t n_rows, qm_status *st,
                                       int sm_count, cudaStream_t stream);
 cudaError_t qm_launch_maxabs(const void *p, int dtype, const uint32_t *nulls, int64_t n, unsigned long long *out,

@@ -26,6 +26,8 @@
 #include "qm_launch.h"
 #include "qm_scan.cuh"
 
+#define QM_PART_WQ (QM_TILE_ROWS + 32)  // per-warp queue: a tile's survivors + < 32 left over
+
 #include <algorithm>
 #include <mutex>
 
@@ -92,8 +94,8 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int warps = blockDim.x >> 5;
-  uint32_t *queue = reinterpret_cast<uint32_t *>(smem) + warp * QM_WQ;
-  uint32_t *cnt = reinterpret_cast<uint32_t *>(smem) + warps * QM_WQ;  // parts + 1 counters
+  uint32_t *queue = reinterpret_cast<uint32_t *>(smem) + warp * QM_PART_WQ;
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(smem) + warps * QM_PART_WQ;  // parts + 1 counters
   __shared__ unsigned long long blk_selected;
   const int P1 = ps.parts + 1;
   for (int p = threadIdx.x; p < P1; p += blockDim.x) cnt[p] = 0;
@@ -108,6 +110,10 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   };
   int qn = 0;
   unsigned long long selected = 0;
+  const char *pf_base;
+  int pf_elem;
+  prefetch_column(a.pred, lane, pf_base, pf_elem);
+  uint32_t pf_want = ~0u;
   for (int64_t v = first; v < n_virtual; v += gwarps) {
     const int64_t tile = tile_of(v);
     if (tile >= n_tiles) continue;
@@ -116,8 +122,8 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
     uint32_t m;
     if (a.vec_ok && e0 + QM_TILE_ROWS <= a.n) {
       const int64_t nxt = v + gwarps < n_virtual ? tile_of(v + gwarps) * QM_TILE_ROWS : a.n;
-      if (nxt + QM_TILE_ROWS <= a.n) prefetch_tile_l2(a.pred, nxt, lane);
-      m = eval_pred_contig(a.pred, r0, (1u << QM_R) - 1);
+      if (nxt + QM_TILE_ROWS <= a.n) prefetch_tile_l2(pf_base, pf_elem, pf_want, nxt, QM_TILE_ROWS, lane);
+      m = eval_pred_contig<1>(a.pred, r0, (1u << QM_R) - 1, pf_want);
     } else {
       int64_t rowv[QM_R];
       m = 0;
@@ -281,7 +287,6 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ qm_scan_args P;
   __shared__ int s_chunk;
-  __shared__ int l_used;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int warps = blockDim.x >> 5;
@@ -321,7 +326,6 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       }
       __syncthreads();
       if (threadIdx.x == 0) {
-        l_used = 0;
         P.priv = 0;
         P.local_rep = 0;
         if (p == ps.parts) {
@@ -371,7 +375,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
         for (int c = 0; c < QM_MAX_VCOLS; ++c) vb[c] = c < QM_NV_BOUND(NV) && c < nv ? w[2 + c] : 0;
         const int special = (int)((w[1] >> 32) & 0xff);
         const uint32_t vnull = (uint32_t)((w[1] >> 40) & 0xff);
-        drain_apply<DD, NV, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, &l_used, lane, active, w[0], special, (uint32_t)w[1],
+        drain_apply<DD, NV, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, lane, active, w[0], special, (uint32_t)w[1],
                                                 vb, vnull);
       }
       __syncthreads();
@@ -399,7 +403,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
 using namespace qm;
 
 size_t qm_part_scan_smem(int parts) {
-  return (size_t)(QM_SCAN_THREADS / 32) * QM_WQ * sizeof(uint32_t) + (size_t)(parts + 1) * sizeof(uint32_t);
+  return (size_t)(QM_SCAN_THREADS / 32) * QM_PART_WQ * sizeof(uint32_t) + (size_t)(parts + 1) * sizeof(uint32_t);
 }
 
 size_t qm_part_agg_smem(int local_slots, int local_hash, int n_words) {
@@ -410,7 +414,7 @@ namespace {
 
 // Kernel attributes and occupancy are set up once per instantiation (the
 // largest shared memory any launch may ask for), not per launch.
-constexpr size_t PART_SCAN_SMEM_MAX = (size_t)(QM_SCAN_THREADS / 32) * QM_WQ * 4 + (size_t)(8192 + 1) * 4;
+constexpr size_t PART_SCAN_SMEM_MAX = (size_t)(QM_SCAN_THREADS / 32) * QM_PART_WQ * 4 + (size_t)(8192 + 1) * 4;
 constexpr size_t PART_AGG_SMEM_MAX = 200 * 1024;
 
 template <auto Kernel>

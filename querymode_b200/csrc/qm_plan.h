@@ -24,6 +24,11 @@
 #define QM_ZONE_TILES 256
 #define QM_ZONE_ROWS (QM_ZONE_TILES * 256)                   // rows per lane per warp tile
 #define QM_TILE_ROWS (QM_R * 32) // rows per warp tile
+// Rows a warp of the scan takes at a time where every warp has enough: two
+// tiles, so that the plan's term fields, the compaction and the loop are paid
+// once for both.
+#define QM_SCAN_TILES 2
+#define QM_SCAN_ROWS (QM_SCAN_TILES * QM_TILE_ROWS)
 
 // ---- predicate terms -------------------------------------------------------
 enum qm_term_kind : int32_t {
@@ -216,6 +221,7 @@ struct qm_outspec {
 };
 
 // ---- one launch of the fused filter + aggregate kernel ----------------------
+#define QM_HEAD_WORDS 3  // accumulator words in the sector of a slot's key
 #define QM_EMPTY_KEY 0x8000000000000000ULL // free hash slot; a real key equal
                                            // to it lives in a reserved slot
 struct qm_status {
@@ -250,7 +256,7 @@ struct qm_staging {
 // (qm_tail_finish): it sorts the groups by first row and writes the result
 // straight into page-locked host memory, where the general path launches a
 // ranking, an emit and three copies.
-#define QM_TAIL_SLOTS 2050   // slots of the table
+#define QM_TAIL_SLOTS 2178   // slots of the table (hashed: 2.1 an estimated group)
 #define QM_TAIL_GROUPS 1024  // groups sorted in shared memory
 struct qm_tail_host {        // page-locked host memory
   qm_status status;
@@ -286,9 +292,8 @@ struct qm_scan_args {
   const uint32_t *sel;   // ascending alive row indices, or null
   int64_t row_offset;    // global index of row 0 (batch order across pushes)
   uint64_t *table;       // group table: slot s = words [s*stride, (s+1)*stride)
-  int64_t n_slots;       // QK_HASH capacity (power of two) / QK_DIRECT size
+  int64_t n_slots;       // QK_HASH capacity / QK_DIRECT size
   int32_t stride;        // 1 key word + agg.n_words
-  int32_t log2cap;       // QK_HASH
   int32_t local_slots;   // block-local table slots (0: none)
   int32_t local_hash;    // block-local table is hashed (else direct-indexed)
   int32_t dedupe;        // warp-level pre-aggregation of equal keys
@@ -299,10 +304,11 @@ struct qm_scan_args {
   int32_t local_rep;     // log2 of the copies of each direct block-local slot
                          // (lane l updates copy l mod copies; local_slots
                          // counts the copies); 0 for hashed or deduplicated
-  int32_t lane_rows;     // rows a lane takes of a tile: 0 as many as QM_R, else
-                         // tiles of 32 * lane_rows rows (few rows: more warps)
+  int32_t lane_rows;     // rows a lane takes at a time: 0 QM_SCAN_TILES * QM_R,
+                         // else 1, 2, 4 or QM_R (few rows: more warps at work)
   int32_t early;         // launched behind qm_tail_init, overlapping its end
-  int32_t pad;
+  int32_t head;          // hash slots are aligned to 32 bytes: the probe reads the
+                         // slot's first three words (QM_HEAD_WORDS) with its key
   const uint32_t *zones; // zones (QM_ZONE_TILES tiles each) to scan, ascending, or null: every tile
   int64_t n_zone_tiles;  // zones: tiles covered (count of zones x QM_ZONE_TILES)
   qm_status *status;

@@ -11,7 +11,15 @@ namespace qm {
 
 // Shared memory of one block: the block-local group table (keys, then the
 // accumulator words structure-of-arrays), then one survivor queue per warp.
-#define QM_WQ (QM_TILE_ROWS + 32)  // per-warp queue: a tile's survivors + < 32 left over
+// Survivors a lane aggregates at once when all have block-local slots: their
+// gathers overlap (200M rows, 16 groups, a third selected: 645 us with one,
+// 578 with two, 556 with four).  Rows that may go to the global table stay at
+// one: their atomics, not their gathers, bound them (100M events 709 us with
+// one, 725 with two, 926 with four).
+#define QM_DRAIN_ROWS 4
+#define QM_WQ (QM_SCAN_ROWS + 32 * QM_DRAIN_ROWS)  // per-warp queue: a tile pair's survivors + those left over
+
+#define QM_LOCAL_TRIAL 32          // drains after which a warp judges the hashed block-local table
 
 struct smem_layout {
   int L;
@@ -49,6 +57,9 @@ __host__ __device__ inline smem_layout make_smem_layout(int local_slots, int loc
 template <bool SEL, bool STAGED, int DD, int NV, int KK, int FT, int LM>
 __global__ void __launch_bounds__(QM_SCAN_THREADS)
     qm_scan_kernel(const __grid_constant__ qm_scan_args a) {
+  constexpr int D = DD == 0 && !SEL && !STAGED && LM == QM_LM_DIRECT && FT >= QM_FT_MIX && NV <= 2
+                        ? (FT == QM_FT_SUM ? QM_DRAIN_ROWS : 2)
+                        : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -66,13 +77,9 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   uint32_t *queue = reinterpret_cast<uint32_t *>(smem + lay.queue_off) + warp * QM_WQ;
   uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + lay.stage_off + warp * lay.stage_warp_bytes);
   uint8_t *sbuf = smem + lay.stage_off + warp * lay.stage_warp_bytes + 32;
-  __shared__ int l_used;
   __shared__ unsigned long long blk_selected;
 
-  if (threadIdx.x == 0) {
-    l_used = 0;
-    blk_selected = 0;
-  }
+  if (threadIdx.x == 0) blk_selected = 0;
   if (L > 0) {
     if (a.local_hash)
       for (int s = threadIdx.x; s < L; s += blockDim.x) lkeys[s] = QM_EMPTY_KEY;
@@ -87,20 +94,51 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();
 
-  const int tile_rows = a.lane_rows ? 32 * a.lane_rows : QM_TILE_ROWS;
-  const int64_t n_tiles = (a.n + tile_rows - 1) / tile_rows;
-  const int64_t full_tiles = a.n / QM_TILE_ROWS;
-  const int64_t gwarps = (int64_t)gridDim.x * warps;
-  const int64_t first = (int64_t)blockIdx.x * warps + warp;
+  // (tile numbers fit 32 bits: rows do)
+  const int tile_rows = STAGED ? QM_TILE_ROWS : (a.lane_rows ? 32 * a.lane_rows : QM_SCAN_ROWS);
+  const int n_tiles = (int)((a.n + tile_rows - 1) / tile_rows);
+  const int full_tiles = (int)(a.n / tile_rows);
+  const int gwarps = (int)gridDim.x * warps;
+  const int first = (int)blockIdx.x * warps + warp;
   const uint32_t lt = lanemask_lt();
   int qn = 0;  // warp-uniform queue length
+  // a hashed block-local table that takes few of a warp's first rows (many
+  // groups, no hot ones) costs more than it saves: that warp leaves it
+  int Lw = L, trial = a.local_hash && L > 0 ? QM_LOCAL_TRIAL : 0, hits = 0;
+  // aggregates queue entries [at, at + count), count <= 32 * D
+  auto drain = [&](int at, int count) {
+    if constexpr (D > 1) {
+      uint32_t row[D];
+      bool act[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        act[d] = d * 32 + lane < count;
+        row[d] = act[d] ? queue[at + d * 32 + lane] : 0;
+      }
+      __syncwarp();
+      drain_rows<NV, KK, FT, D>(a, lwm, L, lane, row, act);
+    } else {
+      const bool act = lane < count;
+      const int64_t row = act ? (int64_t)queue[at + lane] : 0;
+      __syncwarp();
+      const bool hit = drain_round_any<DD, NV, KK, FT, LM>(a, lkeys, lwm, Lw, lane, act, row);
+      if (LM != QM_LM_DIRECT && trial > 0) {
+        hits += __popc(__ballot_sync(QM_FULL, hit));
+        if (--trial == 0 && hits < QM_LOCAL_TRIAL * 32 / 8) Lw = 0;
+      }
+    }
+  };
   unsigned long long selected = 0;
-  int64_t issued = 0;  // STAGED: tiles whose copies were issued (in order)
+  const char *pf_base;  // the filter column this lane prefetches
+  int pf_elem;
+  prefetch_column(a.pred, lane, pf_base, pf_elem);
+  uint32_t pf_want = ~0u;
+  int issued = 0;  // STAGED: tiles whose copies were issued (in order)
   bool failed = false;
 
   // lane 0 issues the copies of the warp's k-th tile into buffer k % depth
-  auto issue = [&](int64_t k) {
-    const int64_t tile = first + k * gwarps;
+  auto issue = [&](int k) {
+    const int64_t tile = first + (int64_t)k * gwarps;
     if (tile >= full_tiles) return;
     if (lane == 0) {
       fence_async_shared();
@@ -114,18 +152,20 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
     issued = k + 1;
   };
   if (STAGED)
-    for (int64_t k = 0; k < S.depth - 1; ++k) issue(k);
+    for (int k = 0; k < S.depth - 1; ++k) issue(k);
 
   // with zone maps, virtual tile v walks the kept zones' tiles
-  const int64_t n_virtual = a.zones ? a.n_zone_tiles : n_tiles;
-  auto tile_of = [&](int64_t v) -> int64_t {
-    return a.zones ? ((int64_t)a.zones[v / QM_ZONE_TILES] * QM_ZONE_TILES + v % QM_ZONE_TILES) : v;
+  // (STAGED and short tiles have none)
+  constexpr int ZONE = QM_ZONE_ROWS / QM_SCAN_ROWS;
+  const int n_virtual = a.zones ? (int)(a.n_zone_tiles / (QM_ZONE_TILES / ZONE)) : n_tiles;
+  auto tile_of = [&](int v) -> int {
+    return a.zones ? (int)(a.zones[v / ZONE] * ZONE + v % ZONE) : v;
   };
-  int64_t k = 0;
-  for (int64_t v = first; v < n_virtual; v += gwarps, ++k) {
-    const int64_t tile = tile_of(v);
+  int k = 0;
+  for (int v = first; v < n_virtual; v += gwarps, ++k) {
+    const int tile = tile_of(v);
     if (tile >= n_tiles) continue;  // the table's last zone is partial
-    const int64_t e0 = tile * tile_rows;
+    const int64_t e0 = (int64_t)tile * tile_rows;
     uint32_t m = 0;
     if (STAGED && tile < full_tiles) {
       __syncwarp();
@@ -148,7 +188,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       const int tot = (int)base - qn;
       qn = (int)base;
       selected += tot;
-    } else if (!SEL && a.lane_rows) {
+    } else if (!SEL && a.lane_rows && a.lane_rows < QM_R) {
       // few rows: short tiles, a row of the warp's 32 per lane and step, so
       // that the serial drains of a tile spread over the idle warps
       for (int j = 0; j < a.lane_rows; ++j) {
@@ -159,15 +199,13 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
         qn += __popc(bal);
         selected += __popc(bal);
       }
-    } else if (!SEL && a.vec_ok && e0 + QM_TILE_ROWS <= a.n) {
-      // full dense tile: the lane's rows are r0 .. r0+7
+    } else if (!SEL && a.vec_ok && e0 + tile_rows <= a.n) {
+      // full dense tiles: the lane's rows are r0 .. r0 + 7 in each
       const int64_t r0 = e0 + (int64_t)lane * QM_R;
-      const int64_t nxt = v + gwarps < n_virtual ? tile_of(v + gwarps) * QM_TILE_ROWS : a.n;
-      if (nxt + QM_TILE_ROWS <= a.n) {
-        prefetch_tile_l2(a.pred, nxt, lane);
-        if (QM_PREFETCH_PAYLOAD) prefetch_payload_l2<NV, KK>(a.key, A, nxt, lane);
-      }
-      m = eval_pred_contig(a.pred, r0, (1u << QM_R) - 1);
+      const int nxt = v + gwarps < n_virtual ? tile_of(v + gwarps) : n_tiles;
+      if (nxt < full_tiles) prefetch_tile_l2(pf_base, pf_elem, pf_want, (int64_t)nxt * tile_rows, tile_rows, lane);
+      m = a.lane_rows ? eval_pred_contig<1>(a.pred, r0, (1u << QM_R) - 1, pf_want)
+                      : eval_pred_contig<QM_SCAN_TILES>(a.pred, r0, (1u << (QM_SCAN_TILES * QM_R)) - 1, pf_want);
       const uint32_t cnt = __popc(m);
       uint32_t off = cnt;
 #pragma unroll
@@ -178,62 +216,51 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       const uint32_t tot = __shfl_sync(QM_FULL, off, 31);
       uint32_t q = qn + off - cnt;
       const uint32_t r0u = (uint32_t)r0;
-      for (uint32_t mm = m; mm; mm &= mm - 1) queue[q++] = r0u + (uint32_t)(__ffs(mm) - 1);
+      for (uint32_t mm = m; mm; mm &= mm - 1) {
+        const uint32_t j = (uint32_t)(__ffs(mm) - 1);
+        queue[q++] = r0u + (j & (QM_R - 1)) + (j / QM_R) * QM_TILE_ROWS;
+      }
       qn += (int)tot;
       selected += tot;
     } else {
-      const int64_t r0 = e0 + (int64_t)lane * QM_R;  // this lane's first element
-      int64_t rowv[QM_R];
+      for (int64_t e1 = e0; e1 < e0 + tile_rows && e1 < a.n; e1 += QM_TILE_ROWS) {
+        const int64_t r0 = e1 + (int64_t)lane * QM_R;  // this lane's first element
+        int64_t rowv[QM_R];
+        m = 0;
 #pragma unroll
-      for (int j = 0; j < QM_R; ++j) {
-        const bool in = r0 + j < a.n;
-        m |= (uint32_t)in << j;
-        rowv[j] = r0 + j;
-      }
-      {
+        for (int j = 0; j < QM_R; ++j) {
+          const bool in = r0 + j < a.n;
+          m |= (uint32_t)in << j;
+          rowv[j] = r0 + j;
+        }
         if (SEL) {
 #pragma unroll
           for (int j = 0; j < QM_R; ++j) rowv[j] = ((m >> j) & 1) ? (int64_t)__ldg(a.sel + r0 + j) : 0;
         }
         auto rowf = [&](int j) { return rowv[j]; };
         m = eval_pred(a.pred, rowf, m);
-      }
-      // append survivors (order inside the queue does not matter: FIRST is a min)
-      const uint32_t cnt = __popc(m);
-      uint32_t off = cnt;
+        // append survivors (order inside the queue does not matter: FIRST is a min)
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t x = __shfl_up_sync(QM_FULL, off, o);
-        if (lane >= o) off += x;
+        for (int j = 0; j < QM_R; ++j) {
+          const uint32_t bal = __ballot_sync(QM_FULL, (m >> j) & 1);
+          if ((m >> j) & 1) queue[qn + __popc(bal & lt)] = (uint32_t)rowv[j];
+          qn += __popc(bal);
+          selected += __popc(bal);
+        }
       }
-      const uint32_t tot = __shfl_sync(QM_FULL, off, 31);
-      off -= cnt;  // exclusive prefix
-      uint32_t q = qn + off;
-#pragma unroll
-      for (int j = 0; j < QM_R; ++j)
-        if ((m >> j) & 1) queue[q++] = (uint32_t)rowv[j];
-      qn += (int)tot;
-      selected += tot;
     }
     __syncwarp();
-    while (qn >= 32) {
-      const int64_t row = queue[qn - 32 + lane];
-      __syncwarp();
-      qn -= 32;
-      drain_round_any<DD, NV, KK, FT, LM>(a, lkeys, lwm, L, &l_used, lane, true, row);
+    while (qn >= 32 * D) {
+      drain(qn - 32 * D, 32 * D);
+      qn -= 32 * D;
     }
   }
   if (STAGED && failed) {
     // let every copy still in flight land before the block's memory goes
-    for (int64_t j = k; j < issued; ++j)
+    for (int j = k; j < issued; ++j)
       if (!mbar_wait(&mbar[j % S.depth], (uint32_t)((j / S.depth) & 1))) break;
   }
-  if (qn > 0) {
-    const bool active = lane < qn;
-    const int64_t row = active ? (int64_t)queue[lane] : 0;
-    __syncwarp();
-    drain_round_any<DD, NV, KK, FT, LM>(a, lkeys, lwm, L, &l_used, lane, active, row);
-  }
+  if (qn > 0) drain(0, qn);
 
   if (lane == 0 && selected) atomicAdd(&blk_selected, selected);
   __syncthreads();
@@ -256,8 +283,11 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
 
 // Launch of one instantiation: `early`, overlapping the end of the clearing
 // launch ahead of it (the kernel waits for it before it touches the table).
+// per_sm non-null: asks how many of its blocks fit an SM instead.
 template <class KERNEL>
-inline cudaError_t launch_scan_kernel(KERNEL kernel, const qm_scan_args &a, int blocks, size_t smem, cudaStream_t st) {
+inline cudaError_t launch_scan_kernel(KERNEL kernel, const qm_scan_args &a, int blocks, size_t smem, cudaStream_t st,
+                                      int *per_sm) {
+  if (per_sm) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, QM_SCAN_THREADS, smem);
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3((unsigned)blocks);
   c.blockDim = dim3(QM_SCAN_THREADS);

@@ -15,13 +15,14 @@
 #if QM_SPEC_NV > 0 && QM_SPEC_NV <= 2
 #define QM_SPEC_SUM(X)                                                                                              \
   X(0, QM_KK_I64, QM_FT_SUM, QM_LM_DIRECT) X(0, QM_KK_I32, QM_FT_SUM, QM_LM_DIRECT)                                 \
-  X(0, QM_KK_I64, QM_FT_SUM, QM_LM_ANY) X(0, QM_KK_I32, QM_FT_SUM, QM_LM_ANY)
+  X(0, QM_KK_I64, QM_FT_SUM, QM_LM_HASH) X(0, QM_KK_I64, QM_FT_SUM, QM_LM_ANY) X(0, QM_KK_I32, QM_FT_SUM, QM_LM_ANY)
 #else
 #define QM_SPEC_SUM(X)
 #endif
 #define QM_SPEC_MIX(X)                                                                                              \
   X(0, QM_KK_I64, QM_FT_MIX, QM_LM_DIRECT) X(0, QM_KK_I32, QM_FT_MIX, QM_LM_DIRECT)                                 \
   X(0, QM_KK_NONE, QM_FT_MIX, QM_LM_DIRECT) X(0, QM_KK_ANY, QM_FT_MIX, QM_LM_DIRECT)                                \
+  X(0, QM_KK_I64, QM_FT_MIX, QM_LM_HASH) X(0, QM_KK_ANY, QM_FT_MIX, QM_LM_HASH)                                     \
   X(0, QM_KK_I64, QM_FT_MIX, QM_LM_ANY) X(0, QM_KK_I32, QM_FT_MIX, QM_LM_ANY)
 #define QM_SPEC_GEN(X)                                                                                              \
   X(0, QM_KK_NONE, QM_FT_GEN, QM_LM_DIRECT) X(0, QM_KK_I64, QM_FT_GEN, QM_LM_ANY)                                   \
@@ -41,11 +42,12 @@ cudaError_t QM_SPEC_FN(_attr)(int max_smem) {
 }
 
 cudaError_t QM_SPEC_FN(_launch)(const qm_scan_args &a, int dd, int kk, int ft, int lm, int blocks, size_t smem,
-                                cudaStream_t st) {
+                                cudaStream_t st, int *per_sm) {
   using namespace qm;
 #define QM_LAUNCH_(DD, KK, FT, LM)                                                                              \
   if (dd == DD && (kk == KK || KK == QM_KK_ANY) && ft >= FT && (lm == LM || LM == QM_LM_ANY)) {                 \
-    return launch_scan_kernel(qm_scan_kernel<false, false, DD, QM_SPEC_NV, KK, FT, LM>, a, blocks, smem, st);    \
+    return launch_scan_kernel(qm_scan_kernel<false, false, DD, QM_SPEC_NV, KK, FT, LM>, a, blocks, smem, st,     \
+                              per_sm);                                                                          \
   }
   QM_SPEC_LIST(QM_LAUNCH_)
 #undef QM_LAUNCH_
