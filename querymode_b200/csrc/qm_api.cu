@@ -1306,20 +1306,64 @@ int table_sel_bound(qm_ctx *ctx, qm_table *t, const qm_pred &P, int64_t *out) {
   return QM_OK;
 }
 
-int column_maxabs(qm_ctx *ctx, DevCol &c, int64_t n) {
-  if (c.has_maxabs) return QM_OK;
-  int rc = ensure(ctx, ctx->counter, 64);
-  if (rc) return rc;
-  rc = ensure_host(ctx, ctx->hstatus, 64);
-  if (rc) return rc;
-  CK(qm_launch_maxabs(c.data, c.dtype, c.nulls, n, (unsigned long long *)ctx->counter.p, ctx->sm_count, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->hstatus.p, ctx->counter.p, 8, cudaMemcpyDeviceToHost, ctx->stream));
+int64_t stat_chunks(int64_t n) { return (n + QM_STAT_ROWS - 1) / QM_STAT_ROWS; }
+
+// A column's statistics from its chunks' (host memory).
+void take_stats(DevCol &c, int64_t n, const qm_chunk_stat *st) {
+  constexpr int64_t PER = QM_ZONE_ROWS / QM_STAT_ROWS;
+  const int64_t chunks = stat_chunks(n), zones = (n + QM_ZONE_ROWS - 1) / QM_ZONE_ROWS;
+  const bool flt = !is_int(c.dtype);
+  auto val = [](int64_t b) {
+    double d;
+    memcpy(&d, &b, 8);
+    return d;
+  };
+  auto less = [&](int64_t x, int64_t y) { return flt ? val(x) < val(y) : x < y; };
+  c.zmin.resize((size_t)zones);
+  c.zmax.resize((size_t)zones);
+  c.zcount.resize((size_t)zones);
+  c.mn = INT64_MAX;
+  c.mx = INT64_MIN;
+  c.maxabs = 0;
+  for (int64_t z = 0; z < zones; z++) {
+    const int64_t k0 = z * PER, k1 = std::min(chunks, k0 + PER);
+    int64_t mn = st[k0].mn, mx = st[k0].mx, cnt = 0;
+    for (int64_t k = k0; k < k1; k++) {
+      if (less(st[k].mn, mn)) mn = st[k].mn;
+      if (less(mx, st[k].mx)) mx = st[k].mx;
+      cnt += st[k].count;
+      c.maxabs = std::max(c.maxabs, val(st[k].maxabs));
+    }
+    c.zmin[z] = mn;
+    c.zmax[z] = mx;
+    c.zcount[z] = cnt;
+    if (!flt) {
+      c.mn = std::min<long long>(c.mn, mn);
+      c.mx = std::max<long long>(c.mx, mx);
+    }
+  }
+  if (flt) c.has_maxabs = true;
+  else c.has_minmax = true;
+  c.has_zones = true;
+}
+
+// Statistics of the columns that lack them, in one synchronise.
+int columns_stats(qm_ctx *ctx, const std::vector<DevCol *> &cols, int64_t n) {
+  if (cols.empty()) return QM_OK;
+  const size_t per = (size_t)std::max<int64_t>(stat_chunks(n), 1) * sizeof(qm_chunk_stat);
+  int rc;
+  if ((rc = ensure(ctx, ctx->zstat, per * cols.size())) || (rc = ensure_host(ctx, ctx->hout, per * cols.size()))) return rc;
+  for (size_t i = 0; i < cols.size(); i++)
+    CK(qm_launch_col_stats(cols[i]->data, cols[i]->dtype, cols[i]->nulls, n,
+                           (qm_chunk_stat *)((char *)ctx->zstat.p + per * i), ctx->stream));
+  if (n > 0) CK(cudaMemcpyAsync(ctx->hout.p, ctx->zstat.p, per * cols.size(), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  uint64_t b = *(uint64_t *)ctx->hstatus.p;
-  memcpy(&c.maxabs, &b, 8);
-  c.has_maxabs = true;
+  for (size_t i = 0; i < cols.size(); i++)
+    take_stats(*cols[i], n, (const qm_chunk_stat *)((const char *)ctx->hout.p + per * i));
   return QM_OK;
 }
+
+int column_maxabs(qm_ctx *ctx, DevCol &c, int64_t n) { return c.has_maxabs ? QM_OK : columns_stats(ctx, {&c}, n); }
 
 // Split constants of the float SUM columns of a table query (see qm_vcol),
 // or, for a deterministic query, the unit of their fixed-point sums: with
@@ -1368,20 +1412,7 @@ int plan_split_sums(qm_ctx *ctx, Plan &pl, int64_t n_rows, bool deterministic) {
   return QM_OK;
 }
 
-int column_minmax(qm_ctx *ctx, DevCol &c, int64_t n) {
-  if (c.has_minmax) return QM_OK;
-  int rc = ensure(ctx, ctx->counter, 64);
-  if (rc) return rc;
-  rc = ensure_host(ctx, ctx->hstatus, 64);
-  if (rc) return rc;
-  CK(qm_launch_minmax(c.data, c.dtype, c.nulls, n, (long long *)ctx->counter.p, ctx->sm_count, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->hstatus.p, ctx->counter.p, 16, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  c.mn = ((long long *)ctx->hstatus.p)[0];
-  c.mx = ((long long *)ctx->hstatus.p)[1];
-  c.has_minmax = true;
-  return QM_OK;
-}
+int column_minmax(qm_ctx *ctx, DevCol &c, int64_t n) { return c.has_minmax ? QM_OK : columns_stats(ctx, {&c}, n); }
 
 // Multi-column keys: integer columns as mixed-radix digits of one 64-bit
 // word (NULL is digit 0 of a nullable column) when the column ranges are
@@ -2225,22 +2256,7 @@ namespace {
 // Zone maps of one column, computed on first use and kept on the column
 // (like its min / max): per zone of QM_ZONE_ROWS rows the non-NULL (non-NaN)
 // cells' min, max and count.
-int column_zones(qm_ctx *ctx, DevCol &c, int64_t n) {
-  if (c.has_zones) return QM_OK;
-  const int64_t zones = (n + QM_ZONE_ROWS - 1) / QM_ZONE_ROWS;
-  int rc = ensure(ctx, ctx->zstat, (size_t)std::max<int64_t>(zones, 1) * 24);
-  if (rc) return rc;
-  int64_t *d = (int64_t *)ctx->zstat.p;
-  CK(qm_launch_zone_stats(c.data, c.dtype, c.nulls, n, d, d + zones, d + 2 * zones, ctx->stream));
-  std::vector<int64_t> h((size_t)zones * 3);
-  if (zones) CK(cudaMemcpyAsync(h.data(), d, (size_t)zones * 24, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  c.zmin.assign(h.begin(), h.begin() + zones);
-  c.zmax.assign(h.begin() + zones, h.begin() + 2 * zones);
-  c.zcount.assign(h.begin() + 2 * zones, h.end());
-  c.has_zones = true;
-  return QM_OK;
-}
+int column_zones(qm_ctx *ctx, DevCol &c, int64_t n) { return c.has_zones ? QM_OK : columns_stats(ctx, {&c}, n); }
 
 // Can term t reject every row of zone z?  A row passes t when its cell is
 // NULL and t.null_pass, or when its value passes the test; the zone map
@@ -2405,6 +2421,25 @@ int plan_table_query(qm_ctx *ctx, qm_table *t, const qm_query *q, GroupTable &gt
   est = 1;
   direct_size = 0;
   uint64_t space = 0;
+  // every column statistic the plan will ask for, in one synchronise
+  {
+    std::vector<DevCol *> need;
+    auto want = [&](const DevCol *c, bool have) {
+      DevCol *m = const_cast<DevCol *>(c);
+      if (c && !have && std::find(need.begin(), need.end(), m) == need.end()) need.push_back(m);
+    };
+    for (int i = 0; i < pl.key.n_cols; i++)
+      if (is_int(pl.keycols[i]->dtype)) want(pl.keycols[i], pl.keycols[i]->has_minmax);
+    for (int c = 0; c < pl.agg.n_vcols; c++)
+      if ((pl.agg.vcol[c].flags & VF_SUM) && !is_int(pl.agg.vcol[c].dtype) && pl.vcolsrc[c])
+        want(pl.vcolsrc[c], pl.vcolsrc[c]->has_maxabs);
+    const int nt = pl.pred.n_groups > 0 ? pl.pred.group_end[pl.pred.n_groups - 1] : pl.pred.n_and;
+    if (t->n_rows > 3 * (int64_t)QM_ZONE_ROWS)
+      for (int i = 0; i < nt; i++)
+        for (auto &c : t->cols)
+          if (c.data == pl.pred.t[i].data && !(pl.pred.t[i].kind == QT_TRUE && pl.pred.t[i].null_pass)) want(&c, c.has_zones);
+    if ((rc = columns_stats(ctx, need, t->n_rows))) return rc;
+  }
   if ((rc = plan_key_packing(ctx, pl, t->n_rows, true, &space))) return rc;
   if ((rc = plan_split_sums(ctx, pl, t->n_rows, (q->flags & QM_FLAG_DETERMINISTIC) != 0))) return rc;
   plan_narrow_sums(pl, t->n_rows);
@@ -2638,8 +2673,7 @@ int qm_table_create(qm_ctx *ctx, int64_t n_rows, int32_t n_cols, const qm_column
   // of float columns, zone maps) of host-uploaded columns are computed on a
   // side stream behind each column's copy, while the next columns cross the
   // host link, instead of on the first query with a synchronise each.
-  const int64_t zones = (n_rows + QM_ZONE_ROWS - 1) / QM_ZONE_ROWS;
-  const size_t per = 32 + (size_t)zones * 24;
+  const size_t per = (size_t)stat_chunks(n_rows) * sizeof(qm_chunk_stat);
   bool eager = n_rows >= EAGER_STATS_ROWS;
   HostBuf hs;
   if (eager) {
@@ -2669,14 +2703,9 @@ int qm_table_create(qm_ctx *ctx, int64_t n_rows, int32_t n_cols, const qm_column
     t->cols.push_back(c);
     if (eager && !cols[i].on_device) {
       uint8_t *d = (uint8_t *)ctx->ustat.p + per * i;
-      int64_t *z = (int64_t *)(d + 32);
       cudaError_t e = cudaEventRecord(ctx->aux_ev, ctx->stream);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->aux, ctx->aux_ev, 0);
-      if (e == cudaSuccess)
-        e = is_int(c.dtype) ? qm_launch_minmax(c.data, c.dtype, c.nulls, n_rows, (long long *)d, ctx->sm_count, ctx->aux)
-                            : qm_launch_maxabs(c.data, c.dtype, c.nulls, n_rows, (unsigned long long *)(d + 16),
-                                               ctx->sm_count, ctx->aux);
-      if (e == cudaSuccess) e = qm_launch_zone_stats(c.data, c.dtype, c.nulls, n_rows, z, z + zones, z + 2 * zones, ctx->aux);
+      if (e == cudaSuccess) e = qm_launch_col_stats(c.data, c.dtype, c.nulls, n_rows, (qm_chunk_stat *)d, ctx->aux);
       if (e == cudaSuccess) e = cudaMemcpyAsync((uint8_t *)hs.p + per * i, d, per, cudaMemcpyDeviceToHost, ctx->aux);
       if (e != cudaSuccess) return fail(set_err(ctx, QM_ERR_CUDA, "column statistics: %s", cudaGetErrorString(e)));
       staged[i] = 1;
@@ -2687,21 +2716,7 @@ int qm_table_create(qm_ctx *ctx, int64_t n_rows, int32_t n_cols, const qm_column
   if (e != cudaSuccess) return fail(set_err(ctx, QM_ERR_CUDA, "upload: %s", cudaGetErrorString(e)));
   for (int i = 0; i < n_cols; i++) {
     if (!staged[i]) continue;
-    DevCol &c = t->cols[i];
-    const uint8_t *h = (const uint8_t *)hs.p + per * i;
-    if (is_int(c.dtype)) {
-      memcpy(&c.mn, h, 8);
-      memcpy(&c.mx, h + 8, 8);
-      c.has_minmax = true;
-    } else {
-      memcpy(&c.maxabs, h + 16, 8);
-      c.has_maxabs = true;
-    }
-    const int64_t *z = (const int64_t *)(h + 32);
-    c.zmin.assign(z, z + zones);
-    c.zmax.assign(z + zones, z + 2 * zones);
-    c.zcount.assign(z + 2 * zones, z + 3 * zones);
-    c.has_zones = true;
+    take_stats(t->cols[i], n_rows, (const qm_chunk_stat *)((const uint8_t *)hs.p + per * i));
   }
   ctx->pool->release(hs);
   *out = t;

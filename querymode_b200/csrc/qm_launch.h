@@ -54,8 +54,6 @@ cudaError_t qm_exclusive_scan_u32(void *temp, size_t *temp_bytes, const uint32_t
 cudaError_t qm_launch_select_write(int64_t n_tiles, const uint32_t *sel, const uint32_t *masks,
                                    const uint64_t *offsets, uint32_t *out, int64_t max_out, int sm_count,
                                    cudaStream_t st);
-cudaError_t qm_launch_minmax(const void *p, int dtype, const uint32_t *nulls, int64_t n, long long *out,
-                             int sm_count, cudaStream_t st);
 cudaError_t qm_launch_export_partial(const uint64_t *t, int stride, const uint32_t *slots, int64_t G, int64_t n_slots,
                                      int key_mode, const qm_aggspec &A, int64_t row_offset, uint64_t *dst, int sm_count,
                                      cudaStream_t st);
@@ -126,8 +124,9 @@ cudaError_t qm_launch_pq_decode(const uint8_t *chunk, const qm_pq_page *pages, i
                                 int n_runs, const qm_pq_run *iruns, int width, int in_width, int conv, int64_t n_rows, uint32_t *present, uint32_t *counts,
                                 uint64_t *ranks, void *temp, size_t *temp_bytes, unsigned char *out, uint32_t *nulls,
                                 int sm_count, cudaStream_t st);
-cudaError_t qm_launch_zone_stats(const void *p, int dtype, const uint32_t *nulls, int64_t n, int64_t *zmin,
-                                 int64_t *zmax, int64_t *zcount, cudaStream_t st);
+// Statistics of a column, one entry per QM_STAT_ROWS rows.
+cudaError_t qm_launch_col_stats(const void *p, int dtype, const uint32_t *nulls, int64_t n, qm_chunk_stat *out,
+                                cudaStream_t st);
 cudaError_t qm_launch_sample_pred(const qm_pred &P, int64_t n, int n_samples, unsigned long long *count,
                                   cudaStream_t st);
 cudaError_t qm_launch_hll(const qm_keyspec &K, int64_t n, uint32_t *regs, int sm_count, cudaStream_t st);
@@ -135,8 +134,6 @@ cudaError_t qm_launch_rehash(const uint64_t *old_t, int64_t old_cap, int stride,
                              int64_t n_slots, qm_status *st, int sm_count, cudaStream_t stream);
 cudaError_t qm_launch_check_selection(const uint32_t *sel, int64_t n_sel, int64_t n_rows, qm_status *st,
                                       int sm_count, cudaStream_t stream);
-cudaError_t qm_launch_maxabs(const void *p, int dtype, const uint32_t *nulls, int64_t n, unsigned long long *out,
-                             int sm_count, cudaStream_t st);
 
 // Partitioned aggregation (qm_part.cu): the counting pass (pass 0) or the
 // scatter pass (pass 1) over the plan's rows, the per-partition offsets, and

@@ -24,6 +24,14 @@
 #define QM_ZONE_TILES 256
 #define QM_ZONE_ROWS (QM_ZONE_TILES * 256)                   // rows per lane per warp tile
 #define QM_TILE_ROWS (QM_R * 32) // rows per warp tile
+// Column statistics are taken in chunks of this many rows (a divisor of a zone).
+#define QM_STAT_ROWS 8192
+#define QM_STAT_THREADS 256
+struct qm_chunk_stat {
+  int64_t mn, mx;   // integer columns: values; float columns: double bits
+  int64_t count;    // non-NULL cells (floats: that are not NaN)
+  int64_t maxabs;   // float columns: bits of the largest finite |x|
+};
 // Rows a warp of the scan takes at a time where every warp has enough: two
 // tiles, so that the plan's term fields, the compaction and the loop are paid
 // once for both.
