@@ -367,6 +367,16 @@ int qm_filter_select(qm_ctx *ctx, int64_t n_rows, int32_t n_cols,
                      uint32_t *out_indices, int64_t max_out,
                      int64_t *out_count);
 
+/* The same selection as a result of one QM_I32 column "index" (the row
+ * indices as unsigned 32-bit numbers) in page-locked memory that the result
+ * owns: the indices cross by DMA and nothing is sized ahead of the count
+ * (30M rows, 2.2M indices: 0.35 ms against 1.4 ms and more into pageable
+ * memory). */
+int qm_filter_select_result(qm_ctx *ctx, int64_t n_rows, int32_t n_cols,
+                            const qm_column *cols, const qm_query *query,
+                            const uint32_t *selection, int64_t n_selected,
+                            qm_result **out);
+
 /* ---- filter -> GROUP BY without allocating --------------------------------- */
 /* Bytes of the fixed device scratch array behind qm_query_run_noalloc. */
 #define QM_NOALLOC_SCRATCH_BYTES (32u << 20)

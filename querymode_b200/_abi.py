@@ -179,6 +179,8 @@ SIGNATURES = [
     ("qm_filter_select", C.c_int, [_P, C.c_int64, C.c_int32, C.POINTER(QmColumn),
                                    C.POINTER(QmQuery), C.POINTER(C.c_uint32), C.c_int64,
                                    C.POINTER(C.c_uint32), C.c_int64, C.POINTER(C.c_int64)]),
+    ("qm_filter_select_result", C.c_int, [_P, C.c_int64, C.c_int32, C.POINTER(QmColumn), C.POINTER(QmQuery),
+                                          C.POINTER(C.c_uint32), C.c_int64, _PP]),
     ("qm_query_run_noalloc", C.c_int, [_P, C.c_int64, C.c_int32, C.POINTER(QmColumn), C.POINTER(QmQuery),
                                        C.c_int64, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p),
                                        C.POINTER(C.c_int32), C.POINTER(C.c_int64)]),

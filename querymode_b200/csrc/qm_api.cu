@@ -3145,6 +3145,67 @@ int agg_push_env(qm_agg *a, const ColEnv &env, int64_t n_rows, const uint32_t *d
   return QM_OK;
 }
 
+// The passing rows of a batch as one bit per element (ctx->masks) and the
+// tiles' offsets in the selection vector (ctx->offsets); *total of them.
+int select_masks(qm_ctx *ctx, int64_t n_rows, int32_t n_cols, const qm_column *cols, const qm_query *q,
+                 const uint32_t *selection, int64_t n_selected, const uint32_t **dsel_out, int64_t *total) {
+  if (n_rows > 0xffffffffLL) return set_err(ctx, QM_ERR_UNSUPPORTED, "batches are limited to 2^32-1 rows");
+  cudaSetDevice(ctx->device);
+  *total = 0;
+  std::vector<DevCol> dcols;
+  int rc = stage_batch(ctx, n_rows, n_cols, cols, dcols);
+  if (rc) return rc;
+  ColEnv env;
+  for (auto &c : dcols) env.views.push_back({&c, n_rows});
+  qm_pred P;
+  std::vector<const DevCol *> touched;
+  int64_t bpr = 0;
+  if ((rc = build_pred(ctx, q, env, P, bpr, touched))) return rc;
+  const uint32_t *dsel = nullptr;
+  if ((rc = stage_selection(ctx, selection, n_selected, &dsel))) return rc;
+  if (dsel && n_selected > 0) {
+    CK(cudaMemsetAsync(ctx->status.p, 0, sizeof(qm_status), ctx->stream));
+    CK(qm_launch_check_selection(dsel, n_selected, n_rows, (qm_status *)ctx->status.p, ctx->sm_count, ctx->stream));
+    qm_status cst;
+    if ((rc = read_status(ctx, &cst))) return rc;
+    if (cst.error) return set_err(ctx, QM_ERR_INVALID, "selection is not strictly ascending row indices below %lld",
+                                  (long long)n_rows);
+  }
+  *dsel_out = dsel;
+  const int64_t n_elems = selection ? n_selected : n_rows;
+  if (n_elems == 0) return QM_OK;
+  const int64_t n_tiles = (n_elems + QM_TILE_ROWS - 1) / QM_TILE_ROWS;
+  if ((rc = ensure(ctx, ctx->masks, (size_t)n_tiles * QM_R * 4)) || (rc = ensure(ctx, ctx->counts, (size_t)n_tiles * 4 + 4)) ||
+      (rc = ensure(ctx, ctx->offsets, (size_t)(n_tiles + 1) * 8)) || (rc = ensure_host(ctx, ctx->hstatus, 64)))
+    return rc;
+  CK(qm_launch_select_masks(P, n_elems, dsel, (uint32_t *)ctx->masks.p, (uint32_t *)ctx->counts.p, ctx->sm_count,
+                            ctx->stream));
+  size_t tb = 0;
+  CK(qm_exclusive_scan_u32(nullptr, &tb, (uint32_t *)ctx->counts.p, (uint64_t *)ctx->offsets.p, n_tiles + 1,
+                           ctx->stream));
+  if ((rc = ensure(ctx, ctx->sort_temp, tb))) return rc;
+  tb = ctx->sort_temp.bytes;
+  // counts[n_tiles] = 0 so offsets[n_tiles] is the total
+  CK(cudaMemsetAsync((uint32_t *)ctx->counts.p + n_tiles, 0, 4, ctx->stream));
+  CK(qm_exclusive_scan_u32(ctx->sort_temp.p, &tb, (uint32_t *)ctx->counts.p, (uint64_t *)ctx->offsets.p,
+                           n_tiles + 1, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->hstatus.p, (uint64_t *)ctx->offsets.p + n_tiles, 8, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  *total = (int64_t)*(uint64_t *)ctx->hstatus.p;
+  return QM_OK;
+}
+
+// The first n_write entries of that selection vector into host memory.
+int select_copy(qm_ctx *ctx, int64_t n_elems, const uint32_t *dsel, int64_t n_write, uint32_t *out) {
+  int rc = ensure(ctx, ctx->sel_out, (size_t)n_write * 4 + 16);
+  if (rc) return rc;
+  CK(qm_launch_select_write((n_elems + QM_TILE_ROWS - 1) / QM_TILE_ROWS, dsel, (uint32_t *)ctx->masks.p,
+                            (uint64_t *)ctx->offsets.p, (uint32_t *)ctx->sel_out.p, n_write, ctx->sm_count, ctx->stream));
+  CK(cudaMemcpyAsync(out, ctx->sel_out.p, (size_t)n_write * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return QM_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -3411,58 +3472,49 @@ int qm_filter_select(qm_ctx *ctx, int64_t n_rows, int32_t n_cols, const qm_colum
   if (!ctx || !q || !out_count || n_rows < 0 || (n_cols > 0 && !cols) || max_out < 0 || (max_out > 0 && !out_indices) ||
       (selection && n_selected < 0))
     return set_err(ctx, QM_ERR_INVALID, "qm_filter_select: bad arguments");
-  if (n_rows > 0xffffffffLL) return set_err(ctx, QM_ERR_UNSUPPORTED, "batches are limited to 2^32-1 rows");
-  cudaSetDevice(ctx->device);
   *out_count = 0;
-  std::vector<DevCol> dcols;
-  int rc = stage_batch(ctx, n_rows, n_cols, cols, dcols);
-  if (rc) return rc;
-  ColEnv env;
-  for (auto &c : dcols) env.views.push_back({&c, n_rows});
-  qm_pred P;
-  std::vector<const DevCol *> touched;
-  int64_t bpr = 0;
-  if ((rc = build_pred(ctx, q, env, P, bpr, touched))) return rc;
+  int64_t total = 0;
   const uint32_t *dsel = nullptr;
-  if ((rc = stage_selection(ctx, selection, n_selected, &dsel))) return rc;
-  if (dsel && n_selected > 0) {
-    CK(cudaMemsetAsync(ctx->status.p, 0, sizeof(qm_status), ctx->stream));
-    CK(qm_launch_check_selection(dsel, n_selected, n_rows, (qm_status *)ctx->status.p, ctx->sm_count, ctx->stream));
-    qm_status cst;
-    if ((rc = read_status(ctx, &cst))) return rc;
-    if (cst.error) return set_err(ctx, QM_ERR_INVALID, "selection is not strictly ascending row indices below %lld",
-                                  (long long)n_rows);
-  }
-  const int64_t n_elems = selection ? n_selected : n_rows;
-  if (n_elems == 0) return QM_OK;
-  const int64_t n_tiles = (n_elems + QM_TILE_ROWS - 1) / QM_TILE_ROWS;
-  if ((rc = ensure(ctx, ctx->masks, (size_t)n_tiles * QM_R * 4)) || (rc = ensure(ctx, ctx->counts, (size_t)n_tiles * 4 + 4)) ||
-      (rc = ensure(ctx, ctx->offsets, (size_t)(n_tiles + 1) * 8)) || (rc = ensure_host(ctx, ctx->hstatus, 64)))
-    return rc;
-  CK(qm_launch_select_masks(P, n_elems, dsel, (uint32_t *)ctx->masks.p, (uint32_t *)ctx->counts.p, ctx->sm_count,
-                            ctx->stream));
-  size_t tb = 0;
-  CK(qm_exclusive_scan_u32(nullptr, &tb, (uint32_t *)ctx->counts.p, (uint64_t *)ctx->offsets.p, n_tiles + 1,
-                           ctx->stream));
-  if ((rc = ensure(ctx, ctx->sort_temp, tb))) return rc;
-  tb = ctx->sort_temp.bytes;
-  // counts[n_tiles] = 0 so offsets[n_tiles] is the total
-  CK(cudaMemsetAsync((uint32_t *)ctx->counts.p + n_tiles, 0, 4, ctx->stream));
-  CK(qm_exclusive_scan_u32(ctx->sort_temp.p, &tb, (uint32_t *)ctx->counts.p, (uint64_t *)ctx->offsets.p,
-                           n_tiles + 1, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->hstatus.p, (uint64_t *)ctx->offsets.p + n_tiles, 8, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  const int64_t total = (int64_t)*(uint64_t *)ctx->hstatus.p;
+  int rc = select_masks(ctx, n_rows, n_cols, cols, q, selection, n_selected, &dsel, &total);
+  if (rc) return rc;
   *out_count = total;
   const int64_t n_write = std::min(total, max_out);
-  if (n_write > 0) {
-    if ((rc = ensure(ctx, ctx->sel_out, (size_t)n_write * 4 + 16))) return rc;
-    CK(qm_launch_select_write(n_tiles, dsel, (uint32_t *)ctx->masks.p, (uint64_t *)ctx->offsets.p,
-                              (uint32_t *)ctx->sel_out.p, n_write, ctx->sm_count, ctx->stream));
-    CK(cudaMemcpyAsync(out_indices, ctx->sel_out.p, (size_t)n_write * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-  }
+  if (n_write > 0 && (rc = select_copy(ctx, selection ? n_selected : n_rows, dsel, n_write, out_indices))) return rc;
   if (total > max_out) return set_err(ctx, QM_ERR_CAPACITY, "%lld rows pass, capacity %lld", (long long)total, (long long)max_out);
+  return QM_OK;
+}
+
+int qm_filter_select_result(qm_ctx *ctx, int64_t n_rows, int32_t n_cols, const qm_column *cols, const qm_query *q,
+                            const uint32_t *selection, int64_t n_selected, qm_result **out) {
+  if (!ctx || !q || !out || n_rows < 0 || (n_cols > 0 && !cols) || (selection && n_selected < 0))
+    return set_err(ctx, QM_ERR_INVALID, "qm_filter_select_result: bad arguments");
+  *out = nullptr;
+  int64_t total = 0;
+  const uint32_t *dsel = nullptr;
+  int rc = select_masks(ctx, n_rows, n_cols, cols, q, selection, n_selected, &dsel, &total);
+  if (rc) return rc;
+  qm_result *R = new qm_result();
+  R->pool = ctx->pool;
+  const size_t bytes = (size_t)total * 4;
+  if (!ctx->pool->acquire(bytes + 16, R->buf)) {
+    delete R;
+    return set_err(ctx, QM_ERR_OOM, "pinned result buffer (%zu bytes)", bytes + 16);
+  }
+  if (total > 0 && (rc = select_copy(ctx, selection ? n_selected : n_rows, dsel, total, (uint32_t *)R->buf.p))) {
+    delete R;
+    return rc;
+  }
+  R->n_rows = total;
+  qm_result::Col c;
+  c.name = "index";
+  c.dtype = QM_I32;
+  c.is_key = 0;
+  c.data = (const uint8_t *)R->buf.p;
+  c.bytes = bytes;
+  R->cols.push_back(std::move(c));
+  R->stats.rows_scanned = selection ? n_selected : n_rows;
+  R->stats.rows_selected = total;
+  *out = R;
   return QM_OK;
 }
 

@@ -1320,14 +1320,30 @@ __global__ void qm_gather_rows(const unsigned char *src, const __grid_constant__
 // Filter-only pass 1: per warp tile, the 32-bit survivor masks and counts.
 template <bool SEL>
 __global__ void __launch_bounds__(QM_SCAN_THREADS)
-    qm_select_masks(const __grid_constant__ qm_pred P, int64_t n, const uint32_t *sel, uint32_t *masks,
+    qm_select_masks(const __grid_constant__ qm_pred P, int64_t n, const uint32_t *sel, bool vec_ok, uint32_t *masks,
                     uint32_t *counts) {
   const int lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   const int64_t n_tiles = (n + QM_TILE_ROWS - 1) / QM_TILE_ROWS;
-  for (int64_t tile = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); tile < n_tiles;
-       tile += (int64_t)gridDim.x * warps) {
+  const int64_t gwarps = (int64_t)gridDim.x * warps;
+  const char *pf_base;
+  int pf_elem;
+  prefetch_column(P, lane, pf_base, pf_elem);
+  uint32_t pf_want = ~0u;
+  for (int64_t tile = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); tile < n_tiles; tile += gwarps) {
     const int64_t e0 = tile * QM_TILE_ROWS;
+    if (!SEL && vec_ok && e0 + QM_TILE_ROWS <= n) {
+      // a lane's eight rows are one byte of the tile's mask (30M rows of two
+      // columns: 93 -> 66 us against a row a lane and step)
+      const int64_t nxt = tile + gwarps;
+      if ((nxt + 1) * QM_TILE_ROWS <= n)
+        prefetch_tile_l2(pf_base, pf_elem, pf_want, nxt * QM_TILE_ROWS, QM_TILE_ROWS, lane);
+      const uint32_t mb = eval_pred_contig<1>(P, e0 + lane * QM_R, (1u << QM_R) - 1, pf_want);
+      reinterpret_cast<uint8_t *>(masks)[tile * QM_TILE_ROWS / 8 + lane] = (uint8_t)mb;
+      const uint32_t c = __reduce_add_sync(QM_FULL, __popc(mb));
+      if (lane == 0) counts[tile] = c;
+      continue;
+    }
     int64_t rowv[QM_R];
     uint32_t m = 0;
 #pragma unroll
@@ -1771,8 +1787,11 @@ cudaError_t qm_launch_select_masks(const qm_pred &P, int64_t n, const uint32_t *
   int warps = QM_SCAN_THREADS / 32;
   int blocks = (int)std::min<int64_t>((n_tiles + warps - 1) / warps, (int64_t)sm_count * 4);
   if (blocks < 1) return cudaSuccess;
-  if (sel) qm_select_masks<true><<<blocks, QM_SCAN_THREADS, 0, st>>>(P, n, sel, masks, counts);
-  else qm_select_masks<false><<<blocks, QM_SCAN_THREADS, 0, st>>>(P, n, sel, masks, counts);
+  const int nt = P.n_groups > 0 ? P.group_end[P.n_groups - 1] : P.n_and;
+  bool vec_ok = true;
+  for (int i = 0; i < nt; ++i) vec_ok = vec_ok && ((uintptr_t)P.t[i].data & 15) == 0;
+  if (sel) qm_select_masks<true><<<blocks, QM_SCAN_THREADS, 0, st>>>(P, n, sel, false, masks, counts);
+  else qm_select_masks<false><<<blocks, QM_SCAN_THREADS, 0, st>>>(P, n, sel, vec_ok, masks, counts);
   return cudaGetLastError();
 }
 

@@ -539,7 +539,7 @@ class Context:
     def filter_select(self, columns: Mapping[str, Any], query: QueryDescriptor,
                       selection: np.ndarray | None = None) -> np.ndarray:
         """Ascending indices of the rows (of `selection`, if given) passing
-        query's filters."""
+        query's filters (a view of page-locked memory the array keeps)."""
         cs = _ColumnSet(columns)
         cq = CQuery(query)
         sel_ptr, n_sel = None, 0
@@ -548,13 +548,17 @@ class Context:
             cs.keep.append(sel)
             sel_ptr = sel.ctypes.data_as(C.POINTER(C.c_uint32))
             n_sel = sel.size
-        cap = n_sel if selection is not None else cs.n_rows
-        out = np.empty(max(cap, 1), dtype=np.uint32)
-        cnt = C.c_int64()
-        self.check(self.lib.qm_filter_select(
-            self.h, cs.n_rows, cs.count, cs.array, cq.ref, sel_ptr, n_sel,
-            out.ctypes.data_as(C.POINTER(C.c_uint32)), cap, C.byref(cnt)))
-        return out[:cnt.value].copy()
+        r = C.c_void_p()
+        self.check(self.lib.qm_filter_select_result(self.h, cs.n_rows, cs.count, cs.array, cq.ref, sel_ptr, n_sel,
+                                                    C.byref(r)))
+        owner = _ResultOwner(self.lib, r)
+        n = C.c_int64()
+        rc = A.QmResultCol()
+        self.lib.qm_result_num_rows(r, C.byref(n))
+        self.lib.qm_result_column(r, 0, C.byref(rc))
+        if n.value == 0:
+            return np.empty(0, dtype=np.uint32)
+        return _buffer_view(rc.data, 4 * n.value, owner).view(np.uint32)
 
     def aggregate(self, query: QueryDescriptor) -> "AggStream":
         return AggStream(self, query)
