@@ -1516,6 +1516,14 @@ struct GroupTable {
   bool small_rank = false;  // ranked in one block (ctx->perm, the count in franks[0])
 };
 
+// The context's copy stream and its events, made on first use.
+int copy_stream(qm_ctx *ctx) {
+  if (ctx->copy) return QM_OK;
+  CK(cudaStreamCreateWithFlags(&ctx->copy, cudaStreamNonBlocking));
+  for (cudaEvent_t &e : ctx->copy_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return QM_OK;
+}
+
 int read_status(qm_ctx *ctx, qm_status *out) {
   int rc = ensure_host(ctx, ctx->hstatus, sizeof(qm_status));
   if (rc) return rc;
@@ -1845,9 +1853,9 @@ int finish_table(qm_ctx *ctx, GroupTable &gt, qm_result **out, float scan_ms_so_
       delete R;
       return rc;
     }
-    if (!ctx->copy) {
-      CK(cudaStreamCreateWithFlags(&ctx->copy, cudaStreamNonBlocking));
-      for (cudaEvent_t &e : ctx->copy_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if ((rc = copy_stream(ctx))) {
+      delete R;
+      return rc;
     }
     qm_scan_args a;
     fill_args(gt, a, (qm_status *)ctx->status.p);
