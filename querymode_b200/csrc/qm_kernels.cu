@@ -1654,8 +1654,10 @@ int key_kind(const qm_keyspec &K) {
   return QM_KK_ANY;
 }
 
+}  // namespace
+
 // The most restricted set of paths (QM_FT_*) the plan's value columns need.
-int value_features(const qm_aggspec &A) {
+int qm_value_features(const qm_aggspec &A) {
   int ft = QM_FT_SUM;
   for (int c = 0; c < A.n_vcols; ++c) {
     const qm_vcol &vc = A.vcol[c];
@@ -1668,7 +1670,6 @@ int value_features(const qm_aggspec &A) {
   }
   return ft;
 }
-}  // namespace
 
 struct scan_choice {
   int dd, kk, ft, lm;
@@ -1679,7 +1680,7 @@ static scan_choice choose_scan(const qm_scan_args &a) {
   scan_choice c;
   c.dd = a.dedupe != 0 ? 1 : 0;
   c.kk = c.dd ? QM_KK_ANY : key_kind(a.key);
-  c.ft = value_features(a.agg);
+  c.ft = qm_value_features(a.agg);
   c.lm = c.dd ? QM_LM_ANY
               : (a.local_slots > 0 && !a.local_hash ? QM_LM_DIRECT : (a.key.mode == QK_HASH && a.head ? QM_LM_HASH : QM_LM_ANY));
   // fixed-point (deterministic) sums run in the run-time-plan kernels only

@@ -144,6 +144,13 @@ cudaError_t qm_launch_part_scan(int pass, const qm_scan_args &a, const qm_part_s
 cudaError_t qm_launch_part_offsets(const qm_part_spec &ps, cudaStream_t st);
 size_t qm_part_agg_smem(int local_slots, int local_hash, int n_words);
 cudaError_t qm_launch_part_agg(const qm_scan_args &a, const qm_part_spec &ps, int sm_count, cudaStream_t st);
+// Windows of a direct table (qm_win_spec): whether the plan's value columns
+// have kernels for it, the scattering block's shared memory, and the four
+// launches (count, offsets, scatter, aggregate).
+int qm_value_features(const qm_aggspec &A);  // QM_FT_*
+bool qm_win_supported(const qm_aggspec &A);
+size_t qm_win_scatter_smem(int windows, int n_vcols);
+cudaError_t qm_launch_windows(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st);
 
 // The library's exclusive scan: scratch bytes for n inputs, and ranks of a
 // bitmap (ranks[i] = set bits in words before i, ranks[words] = all of them).

@@ -398,6 +398,328 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   }
 }
 
+// ---- windows of a large direct table (qm_win_spec) --------------------------------
+// The fused scan updates such a table with four or more reductions a row,
+// bound by the L2's rate for them (85 G/s).  Here a row costs one record
+// written and read (8 bytes and 8 a value column), and its updates are
+// shared-memory atomics.  200M rows, 16.7M slots (4,096 windows), key and one
+// value column: count 0.49 ms, scatter 3.0, aggregation 1.05, against 9.2 ms
+// of key-range passes of the scan.
+
+// The slots of the warp tile of 256 rows at e0: rows e0 + 32 * j + lane that
+// pass (slot[j], or QM_NO_SLOT).  Returns the rows that passed (all lanes').
+#define QM_NO_SLOT 0xffffffffu
+template <int KK>
+__device__ __forceinline__ int win_slots(const qm_scan_args &a, int64_t e0, int lane, uint32_t (&slot)[QM_R]) {
+  uint32_t m;
+  const int64_t r0 = e0 + (int64_t)lane * QM_R;
+  if (a.vec_ok && e0 + QM_TILE_ROWS <= a.n) {
+    uint32_t want;
+    m = eval_pred_contig<1>(a.pred, r0, (1u << QM_R) - 1, want);
+  } else {
+    int64_t rowv[QM_R];
+    m = 0;
+#pragma unroll
+    for (int j = 0; j < QM_R; ++j) {
+      m |= (uint32_t)(r0 + j < a.n) << j;
+      rowv[j] = r0 + j;
+    }
+    auto rowf = [&](int j) { return rowv[j]; };
+    m = eval_pred(a.pred, rowf, m);
+  }
+  // lane l's eight rows follow one another; its keys are read 32 rows apart
+  uint64_t key[QM_R];
+  int special[QM_R];
+  uint32_t pass = 0;
+#pragma unroll
+  for (int j = 0; j < QM_R; ++j) {
+    const uint32_t b = __shfl_sync(QM_FULL, m, j * 4 + (lane >> 3));
+    pass |= ((b >> (lane & 7)) & 1) << j;
+    special[j] = 0;
+    if ((pass >> j) & 1) key[j] = row_key<KK>(a.key, e0 + j * 32 + lane, special[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < QM_R; ++j) {
+    const int64_t s = (pass >> j) & 1 ? global_slot(a, key[j], special[j]) : -1;
+    slot[j] = s >= 0 ? (uint32_t)s : QM_NO_SLOT;
+  }
+  return (int)__reduce_add_sync(QM_FULL, (unsigned)__popc(m));
+}
+
+// Pulls `rows` cells of a column from row r0 on into L2 (one thread).
+__device__ __forceinline__ void win_prefetch(const void *data, int dtype, int64_t r0, int rows) {
+  const int elem = dtype == QM_I32 || dtype == QM_F32 ? 4 : 8;
+  if (((uintptr_t)data & 15) == 0)  // (and r0 is a multiple of 256)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((const char *)data + r0 * elem), "r"(rows * elem) : "memory");
+}
+
+// Records of each window: a block's counts in shared memory, then its totals.
+template <int KK>
+__global__ void __launch_bounds__(QM_SCAN_THREADS)
+    qm_win_count(const __grid_constant__ qm_scan_args a, const __grid_constant__ qm_win_spec ws) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(smem);
+  const int lane = threadIdx.x & 31;
+  const int warps = blockDim.x >> 5;
+  for (int p = threadIdx.x; p < ws.windows; p += blockDim.x) cnt[p] = 0;
+  __syncthreads();
+  const int64_t n_tiles = (a.n + QM_TILE_ROWS - 1) / QM_TILE_ROWS;
+  const int64_t n_virtual = a.zones ? a.n_zone_tiles : n_tiles;
+  unsigned long long selected = 0;
+  for (int64_t v = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); v < n_virtual; v += (int64_t)gridDim.x * warps) {
+    const int64_t tile = a.zones ? (int64_t)a.zones[v / QM_ZONE_TILES] * QM_ZONE_TILES + v % QM_ZONE_TILES : v;
+    if (tile >= n_tiles) continue;
+    uint32_t slot[QM_R];
+    const int64_t nxt = (v + (int64_t)gridDim.x * warps) * QM_TILE_ROWS;
+    if (!a.zones && nxt + QM_TILE_ROWS <= a.n && lane < a.key.n_cols)
+      win_prefetch(a.key.data[lane], a.key.dtype[lane], nxt, QM_TILE_ROWS);
+    selected += win_slots<KK>(a, tile * QM_TILE_ROWS, lane, slot);
+#pragma unroll
+    for (int j = 0; j < QM_R; ++j)
+      if (slot[j] != QM_NO_SLOT) atomicAdd(&cnt[slot[j] >> ws.shift], 1u);
+  }
+  if (lane == 0 && selected) atomicAdd(&a.status->rows_selected, selected);
+  __syncthreads();
+  for (int p = threadIdx.x; p < ws.windows; p += blockDim.x)
+    if (cnt[p]) atomicAdd(&ws.counts[p], cnt[p]);
+}
+
+// Exclusive prefix of one value a thread over a block of T threads.
+template <int T>
+__device__ __forceinline__ uint32_t win_block_scan(uint32_t v, uint32_t *warp_sums, uint32_t &total) {
+  const int lane = threadIdx.x & 31;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(QM_FULL, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_sums[threadIdx.x >> 5] = x;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    uint32_t w = lane < T / 32 ? warp_sums[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(QM_FULL, w, o);
+      if (lane >= o) w += y;
+    }
+    if (lane < T / 32) warp_sums[lane] = w;
+  }
+  __syncthreads();
+  total = warp_sums[T / 32 - 1];
+  return x - v + (threadIdx.x >= 32 ? warp_sums[(threadIdx.x >> 5) - 1] : 0);
+}
+
+// One block: first records and first chunks of the windows.
+__global__ void __launch_bounds__(QM_WIN_THREADS) qm_win_offsets(const __grid_constant__ qm_win_spec ws) {
+  __shared__ uint32_t sums[32];
+  const int per = (ws.windows + QM_WIN_THREADS - 1) / QM_WIN_THREADS;
+  const int p0 = min(ws.windows, (int)threadIdx.x * per), p1 = min(ws.windows, p0 + per);
+  uint32_t n = 0, k = 0;
+  for (int p = p0; p < p1; ++p) {
+    n += ws.counts[p];
+    k += (uint32_t)((ws.counts[p] + ws.chunk - 1) / ws.chunk);
+  }
+  uint32_t n_all, k_all;
+  uint32_t b = win_block_scan<QM_WIN_THREADS>(n, sums, n_all);
+  __syncthreads();
+  uint32_t i = win_block_scan<QM_WIN_THREADS>(k, sums, k_all);
+  for (int p = p0; p < p1; ++p) {
+    ws.bases[p] = ws.cursor[p] = b;
+    ws.items[p] = i;
+    b += ws.counts[p];
+    i += (uint32_t)((ws.counts[p] + ws.chunk - 1) / ws.chunk);
+  }
+  if (threadIdx.x == 0) {
+    ws.bases[ws.windows] = n_all;
+    ws.items[ws.windows] = k_all;
+  }
+}
+
+// A block's 8,192 rows ordered by window in shared memory, then written to
+// the windows' lists in runs (places claimed with one global atomic a window
+// and tile): with 4,096 windows a list's open sector is soon filled by
+// another block, in L2.  Bound by the L2's write requests (36 G/s: records
+// written in row order, without the ordering, 5.6 ms) and, with the runs eight
+// long (1,024 windows, 2.2 ms), by the latency of a tile's phases.  Tiles of
+// 12,288 rows on 768 threads 3.7 ms, 4,096 rows on two blocks of 512 3.4.
+template <int NV, int KK>
+__global__ void __launch_bounds__(QM_WIN_THREADS, 1)
+    qm_win_scatter(const __grid_constant__ qm_scan_args a, const __grid_constant__ qm_win_spec ws) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint32_t sums[32];
+  uint64_t *stage = reinterpret_cast<uint64_t *>(smem);  // [1 + NV][QM_WIN_ROWS]
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(stage + (1 + NV) * QM_WIN_ROWS);  // counts, then first places here
+  uint32_t *delta = cnt + ws.windows;                                            // place in the list less place here
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int64_t n_tiles = (a.n + QM_WIN_ROWS - 1) / QM_WIN_ROWS;
+  constexpr int CLAIMS = 4;
+  constexpr int ZT = QM_ZONE_ROWS / QM_WIN_ROWS;  // block tiles of a zone
+  const int64_t n_virtual = a.zones ? a.n_zone_tiles / QM_ZONE_TILES * ZT : n_tiles;
+  const int per = (ws.windows + QM_WIN_THREADS - 1) / QM_WIN_THREADS;
+  const int p0 = min(ws.windows, (int)threadIdx.x * per), p1 = min(ws.windows, p0 + per);
+  for (int p = threadIdx.x; p < ws.windows; p += blockDim.x) cnt[p] = 0;
+  __syncthreads();
+  for (int64_t v = blockIdx.x; v < n_virtual; v += gridDim.x) {
+    const int64_t tile = a.zones ? (int64_t)a.zones[v / ZT] * ZT + v % ZT : v;
+    if (tile >= n_tiles) continue;  // (the whole block)
+    const int64_t e0 = tile * QM_WIN_ROWS + warp * QM_TILE_ROWS;
+    uint32_t slot[QM_R], rank[QM_R];
+    win_slots<KK>(a, e0, lane, slot);
+#pragma unroll
+    for (int j = 0; j < QM_R; ++j)
+      if (slot[j] != QM_NO_SLOT) rank[j] = atomicAdd(&cnt[slot[j] >> ws.shift], 1u);
+    __syncthreads();
+    // the columns would stand idle until this tile is written out
+    const int64_t nxt = (v + gridDim.x) * QM_WIN_ROWS;
+    if (!a.zones && nxt + QM_WIN_ROWS <= a.n) {
+      if ((int)threadIdx.x < a.key.n_cols) win_prefetch(a.key.data[threadIdx.x], a.key.dtype[threadIdx.x], nxt, QM_WIN_ROWS);
+      else if (threadIdx.x >= 32 && threadIdx.x < 32 + NV)
+        win_prefetch(a.agg.vcol[threadIdx.x - 32].data, a.agg.vcol[threadIdx.x - 32].dtype, nxt, QM_WIN_ROWS);
+    }
+    uint32_t n = 0, total;
+    for (int p = p0; p < p1; ++p) n += cnt[p];
+    uint32_t at = win_block_scan<QM_WIN_THREADS>(n, sums, total);
+    for (int p = p0; p < p1; ++p) {
+      const uint32_t c = cnt[p];
+      delta[p] = c;
+      cnt[p] = at;
+      at += c;
+    }
+    __syncthreads();
+    // the lists' places: neighbouring windows by neighbouring lanes, in
+    // flight while the rows are ordered
+    uint32_t place[CLAIMS];
+#pragma unroll
+    for (int k = 0; k < CLAIMS; ++k) {
+      const int p = (int)threadIdx.x + k * QM_WIN_THREADS;
+      const uint32_t c = p < ws.windows ? delta[p] : 0;
+      if (c) place[k] = atomicAdd(&ws.cursor[p], c);
+    }
+    for (int p = (int)threadIdx.x + CLAIMS * QM_WIN_THREADS; p < ws.windows; p += QM_WIN_THREADS) {
+      const uint32_t c = delta[p];
+      if (c) delta[p] = atomicAdd(&ws.cursor[p], c) - cnt[p];
+    }
+    // four rows' cells in flight (all eight take more registers than there are)
+#pragma unroll
+    for (int j0 = 0; j0 < QM_R; j0 += 4) {
+      uint64_t vb[4][QM_MAX_VCOLS];
+      uint32_t vn[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (slot[j0 + j] != QM_NO_SLOT) gather_values<NV>(a.agg, e0 + (j0 + j) * 32 + lane, vb[j], vn[j]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t s = slot[j0 + j];
+        if (s == QM_NO_SLOT) continue;
+        const uint32_t i = cnt[s >> ws.shift] + rank[j0 + j];
+        stage[i] = (uint64_t)(uint32_t)(e0 + (j0 + j) * 32 + lane) | (uint64_t)s << 32 |
+                   (NV > 0 ? (uint64_t)vn[j] << (32 + QM_WIN_SLOT_BITS) : 0);
+#pragma unroll
+        for (int c = 0; c < NV; ++c) stage[(c + 1) * QM_WIN_ROWS + i] = vb[j][c];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < CLAIMS; ++k) {
+      const int p = (int)threadIdx.x + k * QM_WIN_THREADS;
+      if (p < ws.windows) delta[p] = place[k] - cnt[p];  // (not read where the tile has none)
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < ws.windows; p += blockDim.x) cnt[p] = 0;
+    for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) {
+      const uint64_t w0 = stage[i];
+      const uint32_t p = ((uint32_t)(w0 >> 32) & ((1u << QM_WIN_SLOT_BITS) - 1)) >> ws.shift;
+      const uint32_t to = delta[p] + i;
+      if ((int64_t)to >= ws.rec_cap) {  // the columns changed since they were counted
+        set_error(a.status, QM_DEV_OVERFLOW);
+        continue;
+      }
+      uint64_t *rec = ws.records + (int64_t)to * (1 + NV);
+      if constexpr (NV == 1) {
+        *reinterpret_cast<ulonglong2 *>(rec) = make_ulonglong2(w0, stage[QM_WIN_ROWS + i]);
+      } else {
+        rec[0] = w0;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) rec[c + 1] = stage[(c + 1) * QM_WIN_ROWS + i];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Blocks claim chunks of the windows' lists and aggregate each in a
+// shared-memory window of the table, four records a thread in flight; a
+// window of one chunk is stored, a larger one's chunks are merged.
+template <int NV, int FT>
+__global__ void __launch_bounds__(QM_WIN_THREADS, 1)
+    qm_win_agg(const __grid_constant__ qm_scan_args a, const __grid_constant__ qm_win_spec ws) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int s_item, s_window;
+  const qm_aggspec &A = a.agg;
+  const int L = 1 << ws.shift;
+  uint64_t *lw = reinterpret_cast<uint64_t *>(smem);
+  const int n_items = (int)ws.items[ws.windows];
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const int it = atomicAdd(ws.counter, 1);
+      int lo = 0, hi = ws.windows - 1;  // the last window with items[p] <= it
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if ((int)ws.items[mid] <= it) lo = mid;
+        else hi = mid - 1;
+      }
+      s_item = it;
+      s_window = lo;
+    }
+    for (int i = threadIdx.x; i < L * A.n_words; i += blockDim.x) lw[i] = A.init[i >> ws.shift];
+    __syncthreads();
+    const int it = s_item, p = s_window;
+    if (it >= n_items) break;
+    const int k = it - (int)ws.items[p];
+    const int64_t r0 = (int64_t)ws.bases[p] + k * ws.chunk;
+    const int64_t r1 = min(min((int64_t)ws.bases[p + 1], r0 + ws.chunk), ws.rec_cap);
+    for (int64_t b = r0 + threadIdx.x; b < r1; b += 4 * QM_WIN_THREADS) {
+      uint64_t w[4][1 + NV];
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        const int64_t i = b + d * QM_WIN_THREADS;
+        if (i >= r1) continue;
+        const uint64_t *rec = ws.records + i * (1 + NV);
+        if constexpr (NV == 1) {
+          const ulonglong2 x = __ldcs(reinterpret_cast<const ulonglong2 *>(rec));
+          w[d][0] = x.x;
+          w[d][1] = x.y;
+        } else {
+#pragma unroll
+          for (int c = 0; c <= NV; ++c) w[d][c] = __ldcs(reinterpret_cast<const unsigned long long *>(rec) + c);
+        }
+      }
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        if (b + d * QM_WIN_THREADS >= r1) break;
+        const uint32_t slot = (uint32_t)(w[d][0] >> 32) & ((1u << QM_WIN_SLOT_BITS) - 1);
+        uint64_t vb[QM_MAX_VCOLS];
+#pragma unroll
+        for (int c = 0; c < QM_MAX_VCOLS; ++c) vb[c] = c < NV ? w[d][c < NV ? c + 1 : 0] : 0;
+        agg_row_local<NV, FT>(a, lw, L, (int)(slot & (L - 1)), (uint64_t)a.key.base + slot, slot >= a.n_slots ? 2 : 0,
+                              (uint32_t)w[d][0], vb, (uint32_t)(w[d][0] >> (32 + QM_WIN_SLOT_BITS)));
+      }
+    }
+    __syncthreads();
+    const bool whole = ws.items[p + 1] - ws.items[p] == 1;
+    const int64_t s0 = (int64_t)p << ws.shift;
+    const int slots = (int)min((int64_t)L, ws.total_slots - s0);
+    for (int s = threadIdx.x; s < slots; s += blockDim.x) {
+      if (*limb(lw, L, A.w_count, s) == 0) continue;
+      uint64_t *gp = a.table + (s0 + s) * a.stride + 1;
+      if (whole) store_local(A, lw, L, s, gp, false, a.row_offset);
+      else merge_local(A, lw, L, s, gp, a.row_offset);
+    }
+    __syncthreads();
+  }
+}
+
 }  // namespace qm
 
 using namespace qm;
@@ -521,4 +843,67 @@ cudaError_t qm_launch_part_agg(const qm_scan_args &a, const qm_part_spec &ps, in
   if (!fixed && a.agg.n_vcols == 2)
     return dd ? part_agg_one<1, 2>(a, ps, sm_count, st) : part_agg_one<0, 2>(a, ps, sm_count, st);
   return dd ? part_agg_one<1, QM_NV_ANY>(a, ps, sm_count, st) : part_agg_one<0, QM_NV_ANY>(a, ps, sm_count, st);
+}
+
+// ---- windows of a large direct table ----------------------------------------------
+
+namespace {
+template <int KK>
+cudaError_t win_count(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
+  cudaError_t e = set_smem_once<qm_win_count<KK>>((size_t)QM_WIN_MAX * 4);
+  if (e != cudaSuccess) return e;
+  qm_win_count<KK><<<sm_count * 2, QM_SCAN_THREADS, (size_t)ws.windows * 4, st>>>(a, ws);
+  return cudaGetLastError();
+}
+
+template <int NV, int KK>
+cudaError_t win_scatter(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
+  cudaError_t e = set_smem_once<qm_win_scatter<NV, KK>>(QM_WIN_SMEM_MAX);
+  if (e != cudaSuccess) return e;
+  qm_win_scatter<NV, KK><<<sm_count, QM_WIN_THREADS, qm_win_scatter_smem(ws.windows, NV), st>>>(a, ws);
+  return cudaGetLastError();
+}
+
+template <int NV, int FT>
+cudaError_t win_agg(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
+  cudaError_t e = set_smem_once<qm_win_agg<NV, FT>>(QM_WIN_SMEM_MAX);
+  if (e != cudaSuccess) return e;
+  qm_win_agg<NV, FT><<<sm_count, QM_WIN_THREADS, ((size_t)a.agg.n_words * 8) << ws.shift, st>>>(a, ws);
+  return cudaGetLastError();
+}
+
+template <int NV>
+cudaError_t win_run(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
+  const int kk = part_key_kind(a.key);
+  cudaError_t e = kk == QM_KK_I64   ? win_count<QM_KK_I64>(a, ws, sm_count, st)
+                  : kk == QM_KK_I32 ? win_count<QM_KK_I32>(a, ws, sm_count, st)
+                                    : win_count<QM_KK_ANY>(a, ws, sm_count, st);
+  if (e != cudaSuccess) return e;
+  qm_win_offsets<<<1, QM_WIN_THREADS, 0, st>>>(ws);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  e = kk == QM_KK_I64   ? win_scatter<NV, QM_KK_I64>(a, ws, sm_count, st)
+      : kk == QM_KK_I32 ? win_scatter<NV, QM_KK_I32>(a, ws, sm_count, st)
+                        : win_scatter<NV, QM_KK_ANY>(a, ws, sm_count, st);
+  if (e != cudaSuccess) return e;
+  if constexpr (NV > 0)
+    if (qm_value_features(a.agg) == QM_FT_SUM) return win_agg<NV, QM_FT_SUM>(a, ws, sm_count, st);
+  return win_agg<NV, QM_FT_GEN>(a, ws, sm_count, st);
+}
+}  // namespace
+
+bool qm_win_supported(const qm_aggspec &A) {
+  return A.n_vcols <= QM_WIN_NV_MAX && qm_value_features(A) != QM_FT_FULL;
+}
+
+size_t qm_win_scatter_smem(int windows, int n_vcols) {
+  return (size_t)QM_WIN_ROWS * 8 * (1 + n_vcols) + (size_t)windows * 8;
+}
+
+cudaError_t qm_launch_windows(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
+  if (a.n <= 0) return cudaSuccess;
+  switch (a.agg.n_vcols) {
+    case 0: return win_run<0>(a, ws, sm_count, st);
+    case 1: return win_run<1>(a, ws, sm_count, st);
+    default: return win_run<2>(a, ws, sm_count, st);
+  }
 }

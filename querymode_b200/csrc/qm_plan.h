@@ -349,6 +349,31 @@ struct qm_part_spec {
   int *counter;        // partitions claimed by the aggregating blocks
 };
 
+// ---- windows of a large direct table ---------------------------------------------
+// A direct table of more slots than shared memory holds: every survivor
+// becomes a record in the list of its window (2^shift slots), and a block
+// aggregates a window's records in shared memory.  A record is 1 + n_vcols
+// words: row (bits 0-31), slot (32-57), NULL bits of the cells (58-); the
+// value cells.
+#define QM_WIN_SLOT_BITS 26
+#define QM_WIN_THREADS 1024
+#define QM_WIN_ROWS (QM_WIN_THREADS * QM_R)  // rows a scattering block takes at a time
+#define QM_WIN_NV_MAX 2
+#define QM_WIN_MAX 8448                      // windows of a table (2^25 slots of four words: 8,193)
+#define QM_WIN_SMEM_MAX ((size_t)226 * 1024) // dynamic shared memory of its blocks
+struct qm_win_spec {
+  int32_t windows, shift;
+  int64_t total_slots;
+  int64_t rec_cap;     // records the buffer holds
+  int64_t chunk;       // records a block aggregates at a time (of one window)
+  uint32_t *counts;    // [windows] records of each window (cleared by the caller)
+  uint32_t *cursor;    // [windows] next free record
+  uint32_t *bases;     // [windows + 1] first record
+  uint32_t *items;     // [windows + 1] first chunk
+  int32_t *counter;    // chunks claimed (cleared by the caller)
+  uint64_t *records;
+};
+
 // ---- Parquet column chunk decode (PLAIN pages) --------------------------------
 // A page of a column chunk after its header was parsed on the host.
 struct qm_pq_page {
