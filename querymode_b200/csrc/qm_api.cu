@@ -2418,7 +2418,7 @@ qm_pred with_key_range(const qm_pred &P, const qm_keyspec &K, int64_t lo, int64_
 
 // A direct table of more groups than the scan keeps a block-local table for
 // is aggregated window by window in shared memory (qm_win_spec) where its rows
-// outnumber its slots: scan 9.2 -> 4.5 ms (200M rows, 16.7M slots, key-range
+// outnumber its slots: scan 9.2 -> 3.9 ms (200M rows, 16.7M slots, key-range
 // passes before), 0.31 -> 0.30 (12M rows, 2M slots: the smallest), 61 -> 2.8
 // and 328 -> 3.4 (100M rows, 4.2M slots, Zipf keys and nine rows in ten of one
 // key: reductions on one address).  At 8M rows the two are even (0.23 ms), at

@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
 // bound by the L2's rate for them (85 G/s).  Here a row costs one record
 // written and read (8 bytes and 8 a value column), and its updates are
 // shared-memory atomics.  200M rows, 16.7M slots (4,096 windows), key and one
-// value column: count 0.49 ms, scatter 3.0, aggregation 1.05, against 9.2 ms
+// value column: count 0.42 ms, scatter 2.3, aggregation 1.05, against 9.2 ms
 // of key-range passes of the scan.
 
 // The slots of the warp tile of 256 rows at e0: rows e0 + 32 * j + lane that
@@ -435,13 +435,21 @@ __device__ __forceinline__ int win_slots(const qm_scan_args &a, int64_t e0, int 
   for (int j = 0; j < QM_R; ++j) {
     const uint32_t b = __shfl_sync(QM_FULL, m, j * 4 + (lane >> 3));
     pass |= ((b >> (lane & 7)) & 1) << j;
+    key[j] = 0;
     special[j] = 0;
     if ((pass >> j) & 1) key[j] = row_key<KK>(a.key, e0 + j * 32 + lane, special[j]);
   }
 #pragma unroll
   for (int j = 0; j < QM_R; ++j) {
-    const int64_t s = (pass >> j) & 1 ? global_slot(a, key[j], special[j]) : -1;
-    slot[j] = s >= 0 ? (uint32_t)s : QM_NO_SLOT;
+    // (global_slot of a direct table: its hash branch and a special for keys that
+    // have none spilled the scatter's registers, 3.0 -> 2.3 ms)
+    const uint64_t d = key[j] - (uint64_t)a.key.base;
+    slot[j] = QM_NO_SLOT;
+    if ((pass >> j) & 1) {
+      if (KK == QM_KK_ANY && special[j] == 2) slot[j] = (uint32_t)a.n_slots;
+      else if (d < (uint64_t)a.n_slots) slot[j] = (uint32_t)d;
+      else set_error(a.status, QM_DEV_RANGE);
+    }
   }
   return (int)__reduce_add_sync(QM_FULL, (unsigned)__popc(m));
 }
@@ -541,8 +549,9 @@ __global__ void __launch_bounds__(QM_WIN_THREADS) qm_win_offsets(const __grid_co
 // and tile): with 4,096 windows a list's open sector is soon filled by
 // another block, in L2.  Bound by the L2's write requests (36 G/s: records
 // written in row order, without the ordering, 5.6 ms) and, with the runs eight
-// long (1,024 windows, 2.2 ms), by the latency of a tile's phases.  Tiles of
-// 12,288 rows on 768 threads 3.7 ms, 4,096 rows on two blocks of 512 3.4.
+// long (1,024 windows, 1.8 ms), by the latency of a tile's phases.  While this
+// took 3.0 ms, tiles of 12,288 rows on 768 threads took 3.7 and 4,096 rows on
+// two blocks of 512 3.5.
 template <int NV, int KK>
 __global__ void __launch_bounds__(QM_WIN_THREADS, 1)
     qm_win_scatter(const __grid_constant__ qm_scan_args a, const __grid_constant__ qm_win_spec ws) {
