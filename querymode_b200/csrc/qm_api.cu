@@ -1308,8 +1308,14 @@ int table_sel_bound(qm_ctx *ctx, qm_table *t, const qm_pred &P, int64_t *out) {
 
 int64_t stat_chunks(int64_t n) { return (n + QM_STAT_ROWS - 1) / QM_STAT_ROWS; }
 
-// A column's statistics from its chunks' (host memory).
-void take_stats(DevCol &c, int64_t n, const qm_chunk_stat *st) {
+// The statistics of a column that a plan asks for.
+enum { ST_MINMAX = 1, ST_MAXABS = 2, ST_ZONES = 4, ST_ALL = 7 };
+
+// A column's statistics from its chunks' (host memory).  One pass over the
+// column gives all of them, but of a borrowed column, which its owner may
+// rewrite between queries, only those asked for are kept: the others would be
+// older than the query that first rests on them.
+void take_stats(DevCol &c, int64_t n, const qm_chunk_stat *st, int kinds) {
   constexpr int64_t PER = QM_ZONE_ROWS / QM_STAT_ROWS;
   const int64_t chunks = stat_chunks(n), zones = (n + QM_ZONE_ROWS - 1) / QM_ZONE_ROWS;
   const bool flt = !is_int(c.dtype);
@@ -1319,12 +1325,10 @@ void take_stats(DevCol &c, int64_t n, const qm_chunk_stat *st) {
     return d;
   };
   auto less = [&](int64_t x, int64_t y) { return flt ? val(x) < val(y) : x < y; };
-  c.zmin.resize((size_t)zones);
-  c.zmax.resize((size_t)zones);
-  c.zcount.resize((size_t)zones);
-  c.mn = INT64_MAX;
-  c.mx = INT64_MIN;
-  c.maxabs = 0;
+  if (c.own_data) kinds = ST_ALL;
+  std::vector<int64_t> zmin((size_t)zones), zmax((size_t)zones), zcount((size_t)zones);
+  long long all_mn = INT64_MAX, all_mx = INT64_MIN;
+  double maxabs = 0;
   for (int64_t z = 0; z < zones; z++) {
     const int64_t k0 = z * PER, k1 = std::min(chunks, k0 + PER);
     int64_t mn = st[k0].mn, mx = st[k0].mx, cnt = 0;
@@ -1332,38 +1336,57 @@ void take_stats(DevCol &c, int64_t n, const qm_chunk_stat *st) {
       if (less(st[k].mn, mn)) mn = st[k].mn;
       if (less(mx, st[k].mx)) mx = st[k].mx;
       cnt += st[k].count;
-      c.maxabs = std::max(c.maxabs, val(st[k].maxabs));
+      maxabs = std::max(maxabs, val(st[k].maxabs));
     }
-    c.zmin[z] = mn;
-    c.zmax[z] = mx;
-    c.zcount[z] = cnt;
+    zmin[z] = mn;
+    zmax[z] = mx;
+    zcount[z] = cnt;
     if (!flt) {
-      c.mn = std::min<long long>(c.mn, mn);
-      c.mx = std::max<long long>(c.mx, mx);
+      all_mn = std::min<long long>(all_mn, mn);
+      all_mx = std::max<long long>(all_mx, mx);
     }
   }
-  if (flt) c.has_maxabs = true;
-  else c.has_minmax = true;
-  c.has_zones = true;
+  if (flt && (kinds & ST_MAXABS)) {
+    c.maxabs = maxabs;
+    c.has_maxabs = true;
+  }
+  if (!flt && (kinds & ST_MINMAX)) {
+    c.mn = all_mn;
+    c.mx = all_mx;
+    c.has_minmax = true;
+  }
+  if (kinds & ST_ZONES) {
+    c.zmin = std::move(zmin);
+    c.zmax = std::move(zmax);
+    c.zcount = std::move(zcount);
+    c.has_zones = true;
+  }
 }
 
+struct StatNeed {
+  DevCol *col;
+  int kinds;  // ST_*
+};
+
 // Statistics of the columns that lack them, in one synchronise.
-int columns_stats(qm_ctx *ctx, const std::vector<DevCol *> &cols, int64_t n) {
+int columns_stats(qm_ctx *ctx, const std::vector<StatNeed> &cols, int64_t n) {
   if (cols.empty()) return QM_OK;
   const size_t per = (size_t)std::max<int64_t>(stat_chunks(n), 1) * sizeof(qm_chunk_stat);
   int rc;
   if ((rc = ensure(ctx, ctx->zstat, per * cols.size())) || (rc = ensure_host(ctx, ctx->hout, per * cols.size()))) return rc;
   for (size_t i = 0; i < cols.size(); i++)
-    CK(qm_launch_col_stats(cols[i]->data, cols[i]->dtype, cols[i]->nulls, n,
+    CK(qm_launch_col_stats(cols[i].col->data, cols[i].col->dtype, cols[i].col->nulls, n,
                            (qm_chunk_stat *)((char *)ctx->zstat.p + per * i), ctx->stream));
   if (n > 0) CK(cudaMemcpyAsync(ctx->hout.p, ctx->zstat.p, per * cols.size(), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   for (size_t i = 0; i < cols.size(); i++)
-    take_stats(*cols[i], n, (const qm_chunk_stat *)((const char *)ctx->hout.p + per * i));
+    take_stats(*cols[i].col, n, (const qm_chunk_stat *)((const char *)ctx->hout.p + per * i), cols[i].kinds);
   return QM_OK;
 }
 
-int column_maxabs(qm_ctx *ctx, DevCol &c, int64_t n) { return c.has_maxabs ? QM_OK : columns_stats(ctx, {&c}, n); }
+int column_maxabs(qm_ctx *ctx, DevCol &c, int64_t n) {
+  return c.has_maxabs ? QM_OK : columns_stats(ctx, {{&c, ST_MAXABS}}, n);
+}
 
 // Split constants of the float SUM columns of a table query (see qm_vcol),
 // or, for a deterministic query, the unit of their fixed-point sums: with
@@ -1412,7 +1435,9 @@ int plan_split_sums(qm_ctx *ctx, Plan &pl, int64_t n_rows, bool deterministic) {
   return QM_OK;
 }
 
-int column_minmax(qm_ctx *ctx, DevCol &c, int64_t n) { return c.has_minmax ? QM_OK : columns_stats(ctx, {&c}, n); }
+int column_minmax(qm_ctx *ctx, DevCol &c, int64_t n) {
+  return c.has_minmax ? QM_OK : columns_stats(ctx, {{&c, ST_MINMAX}}, n);
+}
 
 // Multi-column keys: integer columns as mixed-radix digits of one 64-bit
 // word (NULL is digit 0 of a nullable column) when the column ranges are
@@ -2264,7 +2289,9 @@ namespace {
 // Zone maps of one column, computed on first use and kept on the column
 // (like its min / max): per zone of QM_ZONE_ROWS rows the non-NULL (non-NaN)
 // cells' min, max and count.
-int column_zones(qm_ctx *ctx, DevCol &c, int64_t n) { return c.has_zones ? QM_OK : columns_stats(ctx, {&c}, n); }
+int column_zones(qm_ctx *ctx, DevCol &c, int64_t n) {
+  return c.has_zones ? QM_OK : columns_stats(ctx, {{&c, ST_ZONES}}, n);
+}
 
 // Can term t reject every row of zone z?  A row passes t when its cell is
 // NULL and t.null_pass, or when its value passes the test; the zone map
@@ -2506,21 +2533,27 @@ int plan_table_query(qm_ctx *ctx, qm_table *t, const qm_query *q, GroupTable &gt
   uint64_t space = 0;
   // every column statistic the plan will ask for, in one synchronise
   {
-    std::vector<DevCol *> need;
-    auto want = [&](const DevCol *c, bool have) {
-      DevCol *m = const_cast<DevCol *>(c);
-      if (c && !have && std::find(need.begin(), need.end(), m) == need.end()) need.push_back(m);
+    std::vector<StatNeed> need;
+    auto want = [&](const DevCol *c, bool have, int kind) {
+      if (have) return;
+      for (StatNeed &s : need)
+        if (s.col == c) {
+          s.kinds |= kind;
+          return;
+        }
+      need.push_back({const_cast<DevCol *>(c), kind});
     };
     for (int i = 0; i < pl.key.n_cols; i++)
-      if (is_int(pl.keycols[i]->dtype)) want(pl.keycols[i], pl.keycols[i]->has_minmax);
+      if (is_int(pl.keycols[i]->dtype)) want(pl.keycols[i], pl.keycols[i]->has_minmax, ST_MINMAX);
     for (int c = 0; c < pl.agg.n_vcols; c++)
       if ((pl.agg.vcol[c].flags & VF_SUM) && !is_int(pl.agg.vcol[c].dtype) && pl.vcolsrc[c])
-        want(pl.vcolsrc[c], pl.vcolsrc[c]->has_maxabs);
+        want(pl.vcolsrc[c], pl.vcolsrc[c]->has_maxabs, ST_MAXABS);
     const int nt = pl.pred.n_groups > 0 ? pl.pred.group_end[pl.pred.n_groups - 1] : pl.pred.n_and;
     if (t->n_rows > 3 * (int64_t)QM_ZONE_ROWS)
       for (int i = 0; i < nt; i++)
         for (auto &c : t->cols)
-          if (c.data == pl.pred.t[i].data && !(pl.pred.t[i].kind == QT_TRUE && pl.pred.t[i].null_pass)) want(&c, c.has_zones);
+          if (c.data == pl.pred.t[i].data && !(pl.pred.t[i].kind == QT_TRUE && pl.pred.t[i].null_pass))
+            want(&c, c.has_zones, ST_ZONES);
     if ((rc = columns_stats(ctx, need, t->n_rows))) return rc;
   }
   if ((rc = plan_key_packing(ctx, pl, t->n_rows, true, &space))) return rc;
@@ -2799,7 +2832,7 @@ int qm_table_create(qm_ctx *ctx, int64_t n_rows, int32_t n_cols, const qm_column
   if (e != cudaSuccess) return fail(set_err(ctx, QM_ERR_CUDA, "upload: %s", cudaGetErrorString(e)));
   for (int i = 0; i < n_cols; i++) {
     if (!staged[i]) continue;
-    take_stats(t->cols[i], n_rows, (const qm_chunk_stat *)((const uint8_t *)hs.p + per * i));
+    take_stats(t->cols[i], n_rows, (const qm_chunk_stat *)((const uint8_t *)hs.p + per * i), ST_ALL);
   }
   ctx->pool->release(hs);
   *out = t;
