@@ -1135,7 +1135,7 @@ void choose_layout(const Plan &pl, int64_t est_groups, Exec &ex, const qm_tuning
       while ((int64_t)(L * 2) * (per_slot + 8) <= (int64_t)LOCAL_WIDE_BUDGET) L *= 2;
     if (tu.local_slots > 0) {
       L = tu.local_slots;
-      while (L > 4 && (int64_t)L * (per_slot + 8) > (int64_t)200 * 1024) L /= 2;  // fit shared memory
+      while (L > 4 && (int64_t)L * (per_slot + 8) > (int64_t)QM_LOCAL_MAX_BYTES) L /= 2;  // fit shared memory
       L = std::max(L, 4);  // slots are looked up in buckets of four
     }
     ex.local_slots = L;
@@ -1234,8 +1234,6 @@ bool setup_staging(qm_pred &P, qm_staging &S, int depth) {
   S.depth = depth;
   return true;
 }
-
-constexpr size_t SMEM_LIMIT = 227 * 1024;
 
 double hll_estimate(const uint32_t *regs) {
   const int m = 1 << QM_HLL_P;
@@ -2109,7 +2107,7 @@ int scan_args(qm_ctx *ctx, GroupTable &gt, int64_t n, const uint32_t *sel, int b
       if (!setup_staging(a.pred, a.stage, depth)) break;
       size_t sm = qm_scan_smem_bytes(gt.ex.local_slots, gt.ex.local_hash, gt.pl.agg.n_words, a.stage.tile_bytes, depth,
                                      a.priv);
-      if (sm <= SMEM_LIMIT) {
+      if (sm <= (size_t)QM_SCAN_SMEM_MAX) {
         smem = sm;
         staged = true;
       }

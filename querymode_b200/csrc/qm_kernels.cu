@@ -1614,8 +1614,6 @@ size_t qm_scan_smem_bytes(int local_slots, int local_hash, int n_words, int stag
 }
 
 namespace {
-constexpr int QM_SCAN_SMEM_MAX = 227 * 1024 - 1024;  // dynamic, beside the kernel's static words
-
 // Raise every scan kernel's dynamic shared memory limit to the maximum, once
 // per device (launches then pass their actual size).
 cudaError_t scan_attrs_once() {
@@ -1755,7 +1753,9 @@ cudaError_t qm_launch_tail_finish(const qm_tail &T, cudaStream_t st) {
   at.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &at;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, qm_tail_finish, T);
+  const cudaError_t e = cudaLaunchKernelEx(&c, qm_tail_finish, T);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 cudaError_t qm_launch_compact(const uint64_t *t, int64_t n_slots_total, int stride, int count_word,

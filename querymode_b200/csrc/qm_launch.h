@@ -7,6 +7,10 @@
 #include "qm_plan.h"
 
 #define QM_SCAN_THREADS 512
+// Dynamic shared memory of a scan block at most (beside the kernel's static
+// words), and of that its block-local table.
+#define QM_SCAN_SMEM_MAX (227 * 1024 - 1024)
+#define QM_LOCAL_MAX_BYTES (200 * 1024)
 #define QM_HLL_P 12
 
 // Scan kernels specialised for N = 0..QM_SPEC_NV_MAX value columns

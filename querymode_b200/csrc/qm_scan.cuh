@@ -17,7 +17,15 @@ namespace qm {
 // one: their atomics, not their gathers, bound them (100M events 709 us with
 // one, 725 with two, 926 with four).
 #define QM_DRAIN_ROWS 4
-#define QM_WQ (QM_SCAN_ROWS + 32 * QM_DRAIN_ROWS)  // per-warp queue: a tile pair's survivors + those left over
+// Entries of a warp's queue: a tile's survivors and those left over from
+// before, and both tiles' of a pair unless most of their rows pass (those go
+// in tile by tile).  26 KB a block, so that block-local tables of 80 KB leave
+// room for two blocks on an SM, and one of 200 KB fits: room for every pair's
+// rows (640 entries, 40 KB) took the second block from 20M rows into 4,000
+// hashed keys (SUM and COUNT(*), half of the rows: 0.49 ms a query, 0.60 so).
+#define QM_WQ 416
+static_assert(QM_WQ >= QM_TILE_ROWS + 32 * QM_DRAIN_ROWS, "a tile's survivors fit beside those left over");
+static_assert(QM_LOCAL_MAX_BYTES + QM_SCAN_THREADS / 32 * QM_WQ * 4 <= QM_SCAN_SMEM_MAX, "the largest block-local table fits");
 
 #define QM_LOCAL_TRIAL 32          // drains after which a warp judges the hashed block-local table
 
@@ -58,7 +66,7 @@ template <bool SEL, bool STAGED, int DD, int NV, int KK, int FT, int LM>
 __global__ void __launch_bounds__(QM_SCAN_THREADS)
     qm_scan_kernel(const __grid_constant__ qm_scan_args a) {
   constexpr int D = DD == 0 && !SEL && !STAGED && LM == QM_LM_DIRECT && FT >= QM_FT_MIX && NV <= 2
-                        ? (FT == QM_FT_SUM ? QM_DRAIN_ROWS : 2)
+                        ? (FT == QM_FT_SUM || NV == 0 ? QM_DRAIN_ROWS : 2)
                         : 1;
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31;
@@ -166,7 +174,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
     const int tile = tile_of(v);
     if (tile >= n_tiles) continue;  // the table's last zone is partial
     const int64_t e0 = (int64_t)tile * tile_rows;
-    uint32_t m = 0;
+    uint32_t m = 0, left = 0;  // left: rows of m, of all lanes, that are not in the queue yet
     if (STAGED && tile < full_tiles) {
       __syncwarp();
       issue(k + S.depth - 1);
@@ -199,61 +207,65 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
         qn += __popc(bal);
         selected += __popc(bal);
       }
-    } else if (!SEL && a.vec_ok && e0 + tile_rows <= a.n) {
-      // full dense tiles: the lane's rows are r0 .. r0 + 7 in each
-      const int64_t r0 = e0 + (int64_t)lane * QM_R;
-      const int nxt = v + gwarps < n_virtual ? tile_of(v + gwarps) : n_tiles;
-      if (nxt < full_tiles) prefetch_tile_l2(pf_base, pf_elem, pf_want, (int64_t)nxt * tile_rows, tile_rows, lane);
-      m = a.lane_rows ? eval_pred_contig<1>(a.pred, r0, (1u << QM_R) - 1, pf_want)
-                      : eval_pred_contig<QM_SCAN_TILES>(a.pred, r0, (1u << (QM_SCAN_TILES * QM_R)) - 1, pf_want);
-      const uint32_t cnt = __popc(m);
-      uint32_t off = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t x = __shfl_up_sync(QM_FULL, off, o);
-        if (lane >= o) off += x;
-      }
-      const uint32_t tot = __shfl_sync(QM_FULL, off, 31);
-      uint32_t q = qn + off - cnt;
-      const uint32_t r0u = (uint32_t)r0;
-      for (uint32_t mm = m; mm; mm &= mm - 1) {
-        const uint32_t j = (uint32_t)(__ffs(mm) - 1);
-        queue[q++] = r0u + (j & (QM_R - 1)) + (j / QM_R) * QM_TILE_ROWS;
-      }
-      qn += (int)tot;
-      selected += tot;
     } else {
-      for (int64_t e1 = e0; e1 < e0 + tile_rows && e1 < a.n; e1 += QM_TILE_ROWS) {
-        const int64_t r0 = e1 + (int64_t)lane * QM_R;  // this lane's first element
-        int64_t rowv[QM_R];
-        m = 0;
+      if (!SEL && a.vec_ok && e0 + tile_rows <= a.n) {
+        // full dense tiles: the lane's rows are r0 .. r0 + 7 in each
+        const int64_t r0 = e0 + (int64_t)lane * QM_R;
+        const int nxt = v + gwarps < n_virtual ? tile_of(v + gwarps) : n_tiles;
+        if (nxt < full_tiles) prefetch_tile_l2(pf_base, pf_elem, pf_want, (int64_t)nxt * tile_rows, tile_rows, lane);
+        m = a.lane_rows ? eval_pred_contig<1>(a.pred, r0, (1u << QM_R) - 1, pf_want)
+                        : eval_pred_contig<QM_SCAN_TILES>(a.pred, r0, (1u << (QM_SCAN_TILES * QM_R)) - 1, pf_want);
+      } else {
+#pragma unroll 1
+        for (int h = 0; h * QM_TILE_ROWS < tile_rows; ++h) {
+          const int64_t r0 = e0 + h * QM_TILE_ROWS + (int64_t)lane * QM_R;  // this lane's first element
+          int64_t rowv[QM_R];
+          uint32_t mh = 0;
 #pragma unroll
-        for (int j = 0; j < QM_R; ++j) {
-          const bool in = r0 + j < a.n;
-          m |= (uint32_t)in << j;
-          rowv[j] = r0 + j;
-        }
-        if (SEL) {
+          for (int j = 0; j < QM_R; ++j) {
+            const bool in = r0 + j < a.n;
+            mh |= (uint32_t)in << j;
+            rowv[j] = r0 + j;
+          }
+          if (SEL) {
 #pragma unroll
-          for (int j = 0; j < QM_R; ++j) rowv[j] = ((m >> j) & 1) ? (int64_t)__ldg(a.sel + r0 + j) : 0;
-        }
-        auto rowf = [&](int j) { return rowv[j]; };
-        m = eval_pred(a.pred, rowf, m);
-        // append survivors (order inside the queue does not matter: FIRST is a min)
-#pragma unroll
-        for (int j = 0; j < QM_R; ++j) {
-          const uint32_t bal = __ballot_sync(QM_FULL, (m >> j) & 1);
-          if ((m >> j) & 1) queue[qn + __popc(bal & lt)] = (uint32_t)rowv[j];
-          qn += __popc(bal);
-          selected += __popc(bal);
+            for (int j = 0; j < QM_R; ++j) rowv[j] = ((mh >> j) & 1) ? (int64_t)__ldg(a.sel + r0 + j) : 0;
+          }
+          auto rowf = [&](int j) { return rowv[j]; };
+          m |= eval_pred(a.pred, rowf, mh) << (h * QM_R);
         }
       }
+      left = __reduce_add_sync(QM_FULL, __popc(m));
+      selected += left;
     }
-    __syncwarp();
-    while (qn >= 32 * D) {
-      drain(qn - 32 * D, 32 * D);
-      qn -= 32 * D;
-    }
+    do {
+      if (left) {  // (order inside the queue does not matter: FIRST is a min)
+        const uint32_t now = qn + left <= QM_WQ ? m : m & ((1u << QM_R) - 1);
+        m ^= now;
+        const uint32_t cnt = __popc(now);
+        uint32_t off = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t x = __shfl_up_sync(QM_FULL, off, o);
+          if (lane >= o) off += x;
+        }
+        const uint32_t tot = __shfl_sync(QM_FULL, off, 31);
+        uint32_t q = qn + off - cnt;
+        const uint32_t r0u = (uint32_t)(e0 + lane * QM_R);
+        for (uint32_t mm = now; mm; mm &= mm - 1) {
+          const uint32_t j = (uint32_t)(__ffs(mm) - 1);
+          const uint32_t row = r0u + (j & (QM_R - 1)) + (j / QM_R) * QM_TILE_ROWS;
+          queue[q++] = SEL ? __ldg(a.sel + row) : row;
+        }
+        qn += (int)tot;
+        left -= tot;
+      }
+      __syncwarp();
+      while (qn >= 32 * D) {
+        drain(qn - 32 * D, 32 * D);
+        qn -= 32 * D;
+      }
+    } while (left);
   }
   if (STAGED && failed) {
     // let every copy still in flight land before the block's memory goes
@@ -298,7 +310,9 @@ inline cudaError_t launch_scan_kernel(KERNEL kernel, const qm_scan_args &a, int 
   at.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &at;
   c.numAttrs = a.early ? 1 : 0;
-  return cudaLaunchKernelEx(&c, kernel, a);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, a);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next launch
+  return e;
 }
 
 }  // namespace qm
