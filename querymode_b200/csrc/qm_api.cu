@@ -884,6 +884,7 @@ int build_agg(qm_ctx *ctx, const qm_query *q, const ColEnv &env, Plan &pl, std::
     vcols.push_back(c);
     pl.vcolsrc[vcols.size() - 1] = c;
     A.vcol[vcols.size() - 1].split = 0.0;
+    A.vcol[vcols.size() - 1].lim = 0.0;
     A.vcol[vcols.size() - 1].data = c->data;
     A.vcol[vcols.size() - 1].nulls = c->nulls;
     A.vcol[vcols.size() - 1].dtype = c->dtype;
@@ -1397,7 +1398,7 @@ int plan_split_sums(qm_ctx *ctx, Plan &pl, int64_t n_rows, bool deterministic) {
   const int k = bits + 1;  // a group has fewer than 2^(k-1) rows
   for (int c = 0; c < pl.agg.n_vcols; c++) {
     qm_vcol &vc = pl.agg.vcol[c];
-    vc.split = 0.0;
+    vc.split = vc.lim = 0.0;
     if (!(vc.flags & VF_SUM) || is_int(vc.dtype)) continue;
     if (!pl.vcolsrc[c]) {
       if (deterministic) return set_err(ctx, QM_ERR_UNSUPPORTED, "deterministic float SUM needs a registered table");
@@ -1589,6 +1590,10 @@ void fill_args(const GroupTable &gt, qm_scan_args &a, qm_status *st) {
   a.dedupe = gt.ex.dedupe;
   a.priv = gt.ex.priv;
   a.local_rep = gt.ex.local_rep;
+  for (int c = 0; c < gt.pl.agg.n_vcols; c++) {
+    const qm_vcol &vc = gt.pl.agg.vcol[c];
+    if ((vc.flags & VF_SUM) && !(vc.flags & VF_FIXED) && !is_int(vc.dtype) && vc.lim == 0.0) a.doubles = 1;
+  }
   a.zones = gt.zones;
   a.n_zone_tiles = gt.n_zone_tiles;
   a.max_probe = 1 << 12;

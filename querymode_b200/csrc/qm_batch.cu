@@ -160,14 +160,14 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
         const int64_t row = queue[qn - 32 + lane];
         __syncwarp();
         qn -= 32;
-        drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, lane, true, row);
+        drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_DBL)>(P, lkeys, lw, L, lane, true, row);
       }
     }
     if (qn > 0) {
       const bool active = lane < qn;
       const int64_t row = active ? (int64_t)queue[lane] : 0;
       __syncwarp();
-      drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, lane, active, row);
+      drain_round_any<DD, NV, KK, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_DBL)>(P, lkeys, lw, L, lane, active, row);
     }
     __syncthreads();
   }

@@ -1661,8 +1661,10 @@ int qm_value_features(const qm_aggspec &A) {
     const qm_vcol &vc = A.vcol[c];
     const bool isint = vc.dtype == QM_I32 || vc.dtype == QM_I64;
     if (vc.flags & VF_FIXED) return QM_FT_FULL;
-    if (vc.nulls || (vc.flags & (VF_NN | VF_WIDE)) || (!isint && (vc.flags & VF_SUM) && vc.split == 0.0))
-      ft = QM_FT_GEN;
+    if (!isint && (vc.flags & VF_SUM) && vc.lim == 0.0)
+      ft = QM_FT_DBL;
+    else if (vc.nulls || (vc.flags & (VF_NN | VF_WIDE)))
+      ft = ft < QM_FT_GEN ? ft : QM_FT_GEN;
     else if (isint || (vc.flags & (VF_SUM | VF_MIN | VF_MAX | VF_ZERO)) != VF_SUM)
       ft = ft < QM_FT_MIX ? ft : QM_FT_MIX;
   }
@@ -1689,7 +1691,7 @@ static scan_choice choose_scan(const qm_scan_args &a) {
 int qm_scan_kernel_id(const qm_scan_args &a) {
   const scan_choice c = choose_scan(a);
   if (!c.spec) return (c.dd | (a.sel ? 2 : 0) | (a.stage.n > 0 ? 4 : 0));
-  return 8 + (((a.agg.n_vcols * 4 + c.kk) * 4 + c.ft) * 3 + c.lm) * 2 + c.dd;
+  return 8 + (((a.agg.n_vcols * 4 + c.kk) * 5 + c.ft) * 3 + c.lm) * 2 + c.dd;
 }
 
 static cudaError_t scan_dispatch(const qm_scan_args &a, int blocks, size_t smem, cudaStream_t st, int *per_sm) {

@@ -537,14 +537,16 @@ __device__ __forceinline__ bool eval_pred_row(const qm_pred &P, int64_t r, bool 
 #define QM_NV_ANY (QM_MAX_VCOLS + 1)
 #define QM_NV_BOUND(NV) ((NV) > QM_MAX_VCOLS ? QM_MAX_VCOLS : (NV))
 // What the value columns of a plan can need (FT): 0 anything, fixed-point
-// sums included; 1 anything but those; 2 no NULLs, no 128-bit integer sums,
-// float sums split (planned from statistics); 3 as 2, and every column is a
-// float one with a SUM only.  A path a kernel leaves out costs its drain no
-// instructions: the flags are tested once per row and column otherwise.
+// sums included; 1 anything but those; 2 every float sum kept as block-local
+// integers (qm_vcol.lim, planned from statistics); 3 as 2 without NULLs and
+// 128-bit integer sums; 4 as 3, and every column is a float one with a SUM
+// only.  A path a kernel leaves out costs its drain no instructions: the flags
+// are tested once per row and column otherwise.
 #define QM_FT_FULL 0
-#define QM_FT_GEN 1
-#define QM_FT_MIX 2
-#define QM_FT_SUM 3
+#define QM_FT_DBL 1
+#define QM_FT_GEN 2
+#define QM_FT_MIX 3
+#define QM_FT_SUM 4
 // Where rows go (LM): 0 as planned; 1 every row has a slot of the
 // block-local table (a dense key range, or no GROUP BY); 2 a hash table with
 // aligned slots (qm_scan_args.head), through a hashed block-local table or not.
@@ -1211,7 +1213,7 @@ __device__ __forceinline__ void agg_row(const qm_aggspec &A, uint64_t *tp, uint6
           if (stale && st) set_error(st, QM_DEV_STALE);
           if (lo != 0 || hi != 0) add128(w0, w0 + 1, lo, hi);
           if (nf) atomicOr(reinterpret_cast<unsigned long long *>(tp + vc.w_nf), (unsigned long long)nf);
-        } else if (FT >= QM_FT_MIX || vc.split != 0.0) {
+        } else if (FT >= QM_FT_GEN || vc.split != 0.0) {
           split_add(w0, w0 + 1, d, vc.split);
         } else {
           fsum_add(w0, w0 + 1, d, 0.0);
@@ -1246,7 +1248,8 @@ __device__ __forceinline__ void agg_row(const qm_aggspec &A, uint64_t *tp, uint6
 //   split float sum two 64-bit integers in limbs (local_fsum)
 //   fixed-point sum 128 bits in limbs
 // MIN / MAX / FZERO (read first: most rows change nothing), FNF and the
-// TwoSum words of a column without statistics stay 64-bit words at lw[w * L + s].
+// doubles of a column without statistics (local_doubles) stay 64-bit words at
+// lw[w * L + s].
 // Against 64-bit atomics with equal slots merged through __match_any_sync
 // (whole queries, B200): 200M rows into 16 groups 1.23 -> 0.76 ms, 5M rows
 // without GROUP BY 0.29 -> 0.17 ms, 100M events into 65,536 groups 0.78 ->
@@ -1344,7 +1347,7 @@ __device__ __forceinline__ void agg_row_local(const qm_scan_args &a, uint64_t *l
           if (stale) set_error(a.status, QM_DEV_STALE);
           limb_add128(limb(lw, L, vc.w_sum, ls), L, lo, hi);
           if (nf) atomicOr(reinterpret_cast<unsigned long long *>(lw + (int64_t)vc.w_nf * L + ls), (unsigned long long)nf);
-        } else if (FT >= QM_FT_MIX || vc.split != 0.0) {
+        } else if (FT >= QM_FT_GEN || vc.lim != 0.0) {
           double rest;
           const bool in = local_fsum(limb(lw, L, vc.w_sum, ls), L, vc, d, rest);
           if (!in || rest != 0.0) {
@@ -1355,10 +1358,7 @@ __device__ __forceinline__ void agg_row_local(const qm_scan_args &a, uint64_t *l
               else split_add(w0, w0 + 1, d, vc.split);
             }
           }
-        } else {
-          uint64_t *w0 = lw + (int64_t)vc.w_sum * L + ls;
-          fsum_add(w0, w0 + L, d, 0.0);
-        }
+        }  // (sums kept as doubles: local_doubles)
       }
       if (FT <= QM_FT_MIX) {
         if ((f & (VF_MIN | VF_MAX)) && !isnan(d)) {  // NaN never wins '<' / '>'
@@ -1370,6 +1370,48 @@ __device__ __forceinline__ void agg_row_local(const qm_scan_args &a, uint64_t *l
           min_u64(lw + (int64_t)vc.w_zero * L + ls, (((uint64_t)(a.row_offset) + row) << 1) | (vb[c] >> 63));
       }
     }
+  }
+}
+
+// The float sums of the warp's rows that the block-local table keeps as two
+// doubles a slot (columns without statistics: pushed batches).  Lane l's row
+// goes to slot ls (below 0: none); all lanes call this.  An add to a double in
+// shared memory is a compare-and-swap loop, so the lanes of a slot sum theirs
+// first (each takes over its next peer's sum, then that one's: five steps at
+// most) and the lowest adds once, to its warp's copy where slots have copies.
+// 20M rows pushed, half of them kept, SUM and COUNT(*), us of scan against an add
+// a row: one group 2,152 -> 204, 16 502 -> 207, 1,000 371 -> 256.
+template <int NV = QM_NV_ANY>
+__device__ __forceinline__ void local_doubles(const qm_scan_args &a, uint64_t *lw, int L, int ls, int lane,
+                                              const uint64_t (&vb)[QM_MAX_VCOLS], uint32_t vnull) {
+  const qm_aggspec &A = a.agg;
+  const unsigned act = __ballot_sync(QM_FULL, ls >= 0);
+  if (ls < 0) return;
+  const int slot = ls >> a.local_rep;
+  const unsigned peers = __match_any_sync(act, slot);
+  const unsigned above = lane == 31 ? 0u : peers & (~0u << (lane + 1));
+  const bool lowest = lane == __ffs(peers) - 1;
+  const int at = (slot << a.local_rep) | ((int)(threadIdx.x >> 5) & ((1 << a.local_rep) - 1));
+#pragma unroll 1
+  for (int c = 0; c < QM_NV_BOUND(NV); ++c) {
+    if (NV > QM_MAX_VCOLS && c >= A.n_vcols) break;
+    const qm_vcol &vc = A.vcol[c];
+    if (!(vc.flags & VF_SUM) || (vc.flags & VF_FIXED) || vc.lim != 0.0 || vc.dtype == QM_I32 || vc.dtype == QM_I64) continue;
+    double s = (vnull >> c) & 1 ? 0.0 : __longlong_as_double((long long)pick(vb, c)), r = 0.0;
+    bool more = above != 0;
+    int next = more ? __ffs(above) - 1 : lane;
+    while (__any_sync(act, more)) {
+      const double s2 = __shfl_sync(act, s, next), r2 = __shfl_sync(act, r, next);
+      const int n2 = __shfl_sync(act, next, next);
+      if (more) {
+        two_sum_acc(s, r, s2);
+        r += r2;
+      }
+      more = more && n2 != next;  // (the last peer's next is itself)
+      next = more ? n2 : lane;
+    }
+    uint64_t *w0 = lw + (int64_t)vc.w_sum * L + at;
+    if (lowest) fsum_add(w0, w0 + L, s, r);
   }
 }
 
@@ -1453,7 +1495,7 @@ __device__ __forceinline__ void local_load(const qm_aggspec &A, const qm_acc &ac
     case QA_FIRST: v0 = p[0]; break;
     case QA_ISUM:
     case QA_FSUM:
-      if (ac.kind == QA_FSUM && !(A.vcol[ac.vcol].flags & VF_FIXED) && A.vcol[ac.vcol].split == 0.0) {
+      if (ac.kind == QA_FSUM && !(A.vcol[ac.vcol].flags & VF_FIXED) && A.vcol[ac.vcol].lim == 0.0) {
         v0 = lw[(int64_t)ac.word * L + s];
         v1 = lw[(int64_t)(ac.word + 1) * L + s];
       } else {
@@ -1490,7 +1532,7 @@ __device__ __forceinline__ void local_fold(const qm_aggspec &A, const qm_acc &ac
         const uint64_t n = v0 + x0;
         v1 += x1 + (n < v0 ? 1 : 0);
         v0 = n;
-      } else if (A.vcol[ac.vcol].split != 0.0) {
+      } else if (A.vcol[ac.vcol].lim != 0.0) {
         v0 += x0;
         v1 += x1;
       } else {
@@ -1539,7 +1581,7 @@ __device__ __forceinline__ void merge_value(const qm_aggspec &A, const qm_acc &a
     case QA_FSUM:
       if (A.vcol[ac.vcol].flags & VF_FIXED) {
         if (v0 || v1) add128(g0, g1, v0, (int64_t)v1);
-      } else if (A.vcol[ac.vcol].split != 0.0) {
+      } else if (A.vcol[ac.vcol].lim != 0.0) {
         double h, l;
         split_words(A.vcol[ac.vcol], (int64_t)v0, (int64_t)v1, h, l);
         if (h != 0.0) atomicAdd(reinterpret_cast<double *>(g0), h);
@@ -1686,17 +1728,19 @@ __device__ __forceinline__ bool drain_apply(const qm_scan_args &a, uint64_t *lke
                                 local && a.priv, FT == QM_FT_FULL ? a.status : nullptr);
     return false;
   }
+  int ls = -1;
   if (LM == QM_LM_DIRECT) {
     if (active) {
       const int64_t s = global_slot(a, key, special);
-      if (s >= 0)
-        agg_row_local<NV, FT>(a, lw, L, ((int)s << a.local_rep) | (lane & ((1 << a.local_rep) - 1)), key, special, row, vb,
-                              vnull);
+      if (s >= 0) {
+        ls = ((int)s << a.local_rep) | (lane & ((1 << a.local_rep) - 1));
+        agg_row_local<NV, FT>(a, lw, L, ls, key, special, row, vb, vnull);
+      }
     }
     __syncwarp();
+    if (FT <= QM_FT_DBL && a.doubles) local_doubles<NV>(a, lw, L, ls, lane, vb, vnull);
     return false;
   }
-  int ls = -1;
   bool global = active;
   if (L > 0 && active) {
     if (LM != QM_LM_HASH && !a.local_hash) {
@@ -1713,6 +1757,10 @@ __device__ __forceinline__ bool drain_apply(const qm_scan_args &a, uint64_t *lke
   __syncwarp();
   if (ls >= 0) agg_row_local<NV, FT>(a, lw, L, ls, key, special, row, vb, vnull);
   __syncwarp();
+  if (FT <= QM_FT_DBL && a.doubles) {
+    local_doubles<NV>(a, lw, L, ls, lane, vb, vnull);
+    __syncwarp();
+  }
   int64_t gs = -1;
   if constexpr (LM == QM_LM_HASH) {
     slot_head h;

@@ -253,7 +253,7 @@ __device__ __forceinline__ void store_local(const qm_aggspec &A, uint64_t *lw, i
       }
     } else if (ac.kind == QA_FSUM) {
       const qm_vcol &vc = A.vcol[ac.vcol];
-      if (!raw && !(vc.flags & VF_FIXED) && vc.split != 0.0) {
+      if (!raw && !(vc.flags & VF_FIXED) && vc.lim != 0.0) {
         // added, not stored: rare parts of the sum went to these words already
         double h, l;
         split_words(vc, (int64_t)v0, (int64_t)v1, h, l);
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
         for (int c = 0; c < QM_MAX_VCOLS; ++c) vb[c] = c < QM_NV_BOUND(NV) && c < nv ? w[2 + c] : 0;
         const int special = (int)((w[1] >> 32) & 0xff);
         const uint32_t vnull = (uint32_t)((w[1] >> 40) & 0xff);
-        drain_apply<DD, NV, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_GEN)>(P, lkeys, lw, L, lane, active, w[0], special, (uint32_t)w[1],
+        drain_apply<DD, NV, (NV > QM_MAX_VCOLS ? QM_FT_FULL : QM_FT_DBL)>(P, lkeys, lw, L, lane, active, w[0], special, (uint32_t)w[1],
                                                 vb, vnull);
       }
       __syncthreads();
@@ -666,6 +666,7 @@ __global__ void __launch_bounds__(QM_WIN_THREADS, 1)
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_item, s_window;
   const qm_aggspec &A = a.agg;
+  const int lane = threadIdx.x & 31;
   const int L = 1 << ws.shift;
   uint64_t *lw = reinterpret_cast<uint64_t *>(smem);
   const int n_items = (int)ws.items[ws.windows];
@@ -688,7 +689,8 @@ __global__ void __launch_bounds__(QM_WIN_THREADS, 1)
     const int k = it - (int)ws.items[p];
     const int64_t r0 = (int64_t)ws.bases[p] + k * ws.chunk;
     const int64_t r1 = min(min((int64_t)ws.bases[p + 1], r0 + ws.chunk), ws.rec_cap);
-    for (int64_t b = r0 + threadIdx.x; b < r1; b += 4 * QM_WIN_THREADS) {
+    for (int64_t b0 = r0 + (threadIdx.x & ~31u); b0 < r1; b0 += 4 * QM_WIN_THREADS) {  // (whole warps)
+      const int64_t b = b0 + lane;
       uint64_t w[4][1 + NV];
 #pragma unroll
       for (int d = 0; d < 4; ++d) {
@@ -706,13 +708,21 @@ __global__ void __launch_bounds__(QM_WIN_THREADS, 1)
       }
 #pragma unroll
       for (int d = 0; d < 4; ++d) {
-        if (b + d * QM_WIN_THREADS >= r1) break;
+        const bool act = b + d * QM_WIN_THREADS < r1;
+        if (FT > QM_FT_DBL && !act) break;
         const uint32_t slot = (uint32_t)(w[d][0] >> 32) & ((1u << QM_WIN_SLOT_BITS) - 1);
+        const uint32_t vnull = (uint32_t)(w[d][0] >> (32 + QM_WIN_SLOT_BITS));
         uint64_t vb[QM_MAX_VCOLS];
 #pragma unroll
         for (int c = 0; c < QM_MAX_VCOLS; ++c) vb[c] = c < NV ? w[d][c < NV ? c + 1 : 0] : 0;
-        agg_row_local<NV, FT>(a, lw, L, (int)(slot & (L - 1)), (uint64_t)a.key.base + slot, slot >= a.n_slots ? 2 : 0,
-                              (uint32_t)w[d][0], vb, (uint32_t)(w[d][0] >> (32 + QM_WIN_SLOT_BITS)));
+        if (act)
+          agg_row_local<NV, FT>(a, lw, L, (int)(slot & (L - 1)), (uint64_t)a.key.base + slot, slot >= a.n_slots ? 2 : 0,
+                                (uint32_t)w[d][0], vb, vnull);
+        if (FT <= QM_FT_DBL) {
+          __syncwarp();
+          local_doubles<NV>(a, lw, L, act ? (int)(slot & (L - 1)) : -1, lane, vb, vnull);
+          __syncwarp();
+        }
       }
     }
     __syncthreads();
@@ -894,8 +904,11 @@ cudaError_t win_run(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, 
       : kk == QM_KK_I32 ? win_scatter<NV, QM_KK_I32>(a, ws, sm_count, st)
                         : win_scatter<NV, QM_KK_ANY>(a, ws, sm_count, st);
   if (e != cudaSuccess) return e;
-  if constexpr (NV > 0)
-    if (qm_value_features(a.agg) == QM_FT_SUM) return win_agg<NV, QM_FT_SUM>(a, ws, sm_count, st);
+  if constexpr (NV > 0) {
+    const int ft = qm_value_features(a.agg);
+    if (ft == QM_FT_SUM) return win_agg<NV, QM_FT_SUM>(a, ws, sm_count, st);
+    if (ft == QM_FT_DBL) return win_agg<NV, QM_FT_DBL>(a, ws, sm_count, st);
+  }
   return win_agg<NV, QM_FT_GEN>(a, ws, sm_count, st);
 }
 }  // namespace

@@ -168,7 +168,7 @@ struct qm_vcol {
   int32_t w_nf;
   double fx_max;
   // Block-local float SUM of a split column (see local_fsum): a cell below
-  // lim in magnitude is added as two 64-bit integers, in units of ga and gb,
+  // lim (0: kept as two doubles) in magnitude is added as two 64-bit integers, in units of ga and gb,
   // found by adding sa = 1.5 * 2^p and sb = 1.5 * 2^q (ga = 2^(p-52),
   // gb = 2^(q-52)); ulp(split) = ga * 2^lsh.
   double lim, sa, sb, ga, gb;
@@ -317,6 +317,7 @@ struct qm_scan_args {
   int32_t early;         // launched behind qm_tail_init, overlapping its end
   int32_t head;          // hash slots are aligned to 32 bytes: the probe reads the
                          // slot's first three words (QM_HEAD_WORDS) with its key
+  int32_t doubles;       // a float SUM whose block-local words are doubles
   const uint32_t *zones; // zones (QM_ZONE_TILES tiles each) to scan, ascending, or null: every tile
   int64_t n_zone_tiles;  // zones: tiles covered (count of zones x QM_ZONE_TILES)
   qm_status *status;
