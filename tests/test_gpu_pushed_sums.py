@@ -49,25 +49,39 @@ def test_sums(ctx, kind, groups, aggs):
     assert_same(s.finish(), oracle.run(twice, q), ctx_msg=f"twice {kind} {groups} {aggs}")
 
 
-def test_one_group_costs_no_more(ctx):
+def push_times(ctx, keys):
+    """Seconds of a push of SUM and COUNT(*) by each of `keys`."""
     import torch
-    n = 20_000_000
     g = torch.Generator(device="cuda")
     g.manual_seed(1)
-    x = torch.randn(n, generator=g, device="cuda", dtype=torch.float64)
-    many = torch.randint(0, 500, (n,), generator=g, device="cuda")
-    torch.cuda.synchronize()
+    x = torch.randn(len(keys[0]), generator=g, device="cuda", dtype=torch.float64)
     q = QueryDescriptor(group_by=["key"], aggregates=[AggregateOp("sum", "x"), AggregateOp("count", "*")])
-    ms = []
-    for key in (many, torch.zeros_like(many)):
+    out = []
+    for key in keys:
         torch.cuda.synchronize()
         t = ctx.table({"key": key, "x": x})
         best = 1e9
-        for _ in range(4):
+        for _ in range(6):
             s = ctx.aggregate(q)
             t0 = time.perf_counter()
             s.push_table(t)
             best = min(best, time.perf_counter() - t0)
             s.close()
-        ms.append(best)
+        out.append(best)
+    return out
+
+
+def test_one_group_costs_no_more(ctx):
+    import torch
+    many = torch.randint(0, 500, (20_000_000,), device="cuda")
+    ms = push_times(ctx, [many, torch.zeros_like(many)])
     assert ms[1] < 3 * ms[0], ms
+
+
+def test_keys_in_a_row_cost_no_more(ctx):
+    """Sixteen keys that follow one another against sixteen random ones: twice
+    as long while they met on one bank of shared memory."""
+    import torch
+    idx = torch.randint(0, 16, (50_000_000,), device="cuda")
+    ms = push_times(ctx, [torch.randint(-2**62, 2**62, (16,), device="cuda")[idx], idx])
+    assert ms[1] < 1.5 * ms[0], ms
