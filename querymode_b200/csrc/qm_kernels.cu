@@ -807,12 +807,24 @@ __global__ void __launch_bounds__(QM_STAT_THREADS) qm_col_stats(const T *p, cons
       s.cnt += w[i][2];
       ab = max(ab, w[i][3]);
     }
-    qm_chunk_stat r;
+    qm_chunk_stat &r = out[blockIdx.x];
     r.mn = FLT ? __double_as_longlong(ord2f(s.mn)) : s.mn;
     r.mx = FLT ? __double_as_longlong(ord2f(s.mx)) : s.mx;
     r.count = s.cnt;
     r.maxabs = ab;
-    out[blockIdx.x] = r;
+  }
+  if (threadIdx.x < QM_STAT_SAMPLES) {
+    constexpr int STEP = QM_STAT_ROWS / QM_STAT_SAMPLES;
+    const int64_t row = r0 + threadIdx.x * STEP + (blockIdx.x * 0x9e3779b1u >> 16) % STEP;
+    int16_t low = QM_NO_BIT;
+    if (FLT && row < n && !cell_null(nulls, row)) {
+      const double d = (double)p[row];
+      const long long b = __double_as_longlong(d);
+      const int ex = (int)((b >> 52) & 0x7ff);
+      const long long m = (b & ((1LL << 52) - 1)) | (ex ? 1LL << 52 : 0);
+      if (ex != 0x7ff && m != 0) low = (int16_t)((ex ? ex : 1) - 1075 + __ffsll(m) - 1);
+    }
+    out[blockIdx.x].low[threadIdx.x] = low;
   }
 }
 

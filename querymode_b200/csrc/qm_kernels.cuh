@@ -767,11 +767,15 @@ __device__ __forceinline__ void split_parts(double x, double split, double &xh, 
   xl = __dsub_rn(x, xh);
 }
 
+__device__ __forceinline__ void split_words_add(uint64_t *hp, uint64_t *lp, double xh, double xl) {
+  if (xh != 0.0 || isnan(xh)) atomicAdd(reinterpret_cast<double *>(hp), xh);
+  if (xl != 0.0) atomicAdd(reinterpret_cast<double *>(lp), xl);
+}
+
 __device__ __forceinline__ void split_add(uint64_t *hp, uint64_t *lp, double x, double split) {
   double xh, xl;
   split_parts(x, split, xh, xl);
-  if (xh != 0.0 || isnan(xh)) atomicAdd(reinterpret_cast<double *>(hp), xh);
-  if (xl != 0.0) atomicAdd(reinterpret_cast<double *>(lp), xl);
+  split_words_add(hp, lp, xh, xl);
 }
 
 __device__ __forceinline__ void two_sum_acc(double &s, double &c, double x) {
@@ -1257,7 +1261,7 @@ __device__ __forceinline__ void agg_row(const qm_aggspec &A, uint64_t *tp, uint6
 //   split float sum two 64-bit integers in limbs (local_fsum)
 //   fixed-point sum 128 bits in limbs
 // MIN / MAX / FZERO (read first: most rows change nothing), FNF and the
-// doubles of a column without statistics (local_doubles) stay 64-bit words at
+// doubles of local_doubles stay 64-bit words at
 // lw[w * L + s].
 // Against 64-bit atomics with equal slots merged through __match_any_sync
 // (whole queries, B200): 200M rows into 16 groups 1.23 -> 0.76 ms, 5M rows
@@ -1383,7 +1387,8 @@ __device__ __forceinline__ void agg_row_local(const qm_scan_args &a, uint64_t *l
 }
 
 // The float sums of the warp's rows that the block-local table keeps as two
-// doubles a slot (columns without statistics: pushed batches).  Lane l's row
+// doubles a slot (columns without statistics: pushed batches; split columns
+// whose cells differ too much in size for integers: wide_cells).  Lane l's row
 // goes to slot ls (below 0: none); all lanes call this.  An add to a double in
 // shared memory is a compare-and-swap loop, so the lanes of a slot sum theirs
 // first (each takes over its next peer's sum, then that one's: five steps at
@@ -1407,6 +1412,7 @@ __device__ __forceinline__ void local_doubles(const qm_scan_args &a, uint64_t *l
     const qm_vcol &vc = A.vcol[c];
     if (!(vc.flags & VF_SUM) || (vc.flags & VF_FIXED) || vc.lim != 0.0 || vc.dtype == QM_I32 || vc.dtype == QM_I64) continue;
     double s = (vnull >> c) & 1 ? 0.0 : __longlong_as_double((long long)pick(vb, c)), r = 0.0;
+    if (vc.split != 0.0) split_parts(s, vc.split, s, r);
     bool more = above != 0;
     int next = more ? __ffs(above) - 1 : lane;
     while (__any_sync(act, more)) {
@@ -1420,7 +1426,10 @@ __device__ __forceinline__ void local_doubles(const qm_scan_args &a, uint64_t *l
       next = more ? n2 : lane;
     }
     uint64_t *w0 = lw + (int64_t)vc.w_sum * L + at;
-    if (lowest) fsum_add(w0, w0 + L, s, r);
+    if (lowest) {
+      if (vc.split != 0.0) split_words_add(w0, w0 + L, s, r);
+      else fsum_add(w0, w0 + L, s, r);
+    }
   }
 }
 
@@ -1596,7 +1605,9 @@ __device__ __forceinline__ void merge_value(const qm_aggspec &A, const qm_acc &a
         if (h != 0.0) atomicAdd(reinterpret_cast<double *>(g0), h);
         if (l != 0.0) atomicAdd(reinterpret_cast<double *>(g1), l);
       } else {
-        fsum_add(g0, g1, __longlong_as_double((long long)v0), __longlong_as_double((long long)v1));
+        const double h = __longlong_as_double((long long)v0), l = __longlong_as_double((long long)v1);
+        if (A.vcol[ac.vcol].split != 0.0) split_words_add(g0, g1, h, l);
+        else fsum_add(g0, g1, h, l);
       }
       break;
     case QA_IMIN:
