@@ -112,7 +112,8 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
   int qn = 0;  // warp-uniform queue length
   // a hashed block-local table that takes few of a warp's first rows (many
   // groups, no hot ones) costs more than it saves: that warp leaves it
-  int Lw = L, trial = a.local_hash && L > 0 ? QM_LOCAL_TRIAL : 0, hits = 0;
+  // (deduplicating plans keep it: their rows are merged ahead of the lookup)
+  int Lw = L, trial = DD == 0 && a.local_hash && L > 0 ? QM_LOCAL_TRIAL : 0, hits = 0;
   // aggregates queue entries [at, at + count), count <= 32 * D
   auto drain = [&](int at, int count) {
     if constexpr (D > 1) {
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
       const int64_t row = act ? (int64_t)queue[at + lane] : 0;
       __syncwarp();
       const bool hit = drain_round_any<DD, NV, KK, FT, LM>(a, lkeys, lwm, Lw, lane, act, row);
-      if (LM != QM_LM_DIRECT && trial > 0) {
+      if (DD == 0 && LM != QM_LM_DIRECT && trial > 0) {
         hits += __popc(__ballot_sync(QM_FULL, hit));
         if (--trial == 0 && hits < QM_LOCAL_TRIAL * 32 / 8) Lw = 0;
       }
