@@ -26,9 +26,11 @@
   X(0, QM_KK_I64, QM_FT_MIX, QM_LM_ANY) X(0, QM_KK_I32, QM_FT_MIX, QM_LM_ANY)
 #if QM_SPEC_NV > 0
 #define QM_SPEC_GEN(X)                                                                                              \
-  X(0, QM_KK_NONE, QM_FT_GEN, QM_LM_DIRECT) X(0, QM_KK_I64, QM_FT_GEN, QM_LM_ANY)                                   \
-  X(0, QM_KK_I32, QM_FT_GEN, QM_LM_ANY) X(0, QM_KK_ANY, QM_FT_GEN, QM_LM_ANY)                                       \
-  X(0, QM_KK_NONE, QM_FT_DBL, QM_LM_DIRECT) X(0, QM_KK_I64, QM_FT_DBL, QM_LM_ANY)                                   \
+  X(0, QM_KK_NONE, QM_FT_GEN, QM_LM_DIRECT)                                                                         \
+  X(0, QM_KK_I64, QM_FT_GEN, QM_LM_HASH) X(0, QM_KK_ANY, QM_FT_GEN, QM_LM_HASH)                                     \
+  X(0, QM_KK_I64, QM_FT_GEN, QM_LM_ANY) X(0, QM_KK_I32, QM_FT_GEN, QM_LM_ANY) X(0, QM_KK_ANY, QM_FT_GEN, QM_LM_ANY) \
+  X(0, QM_KK_NONE, QM_FT_DBL, QM_LM_DIRECT)                                                                         \
+  X(0, QM_KK_I64, QM_FT_DBL, QM_LM_HASH) X(0, QM_KK_ANY, QM_FT_DBL, QM_LM_HASH) X(0, QM_KK_I64, QM_FT_DBL, QM_LM_ANY) \
   X(0, QM_KK_I32, QM_FT_DBL, QM_LM_ANY) X(0, QM_KK_ANY, QM_FT_DBL, QM_LM_ANY) X(1, QM_KK_ANY, QM_FT_DBL, QM_LM_ANY)
 #else
 #define QM_SPEC_GEN(X) X(0, QM_KK_ANY, QM_FT_GEN, QM_LM_ANY) X(1, QM_KK_ANY, QM_FT_GEN, QM_LM_ANY)
