@@ -2514,6 +2514,11 @@ bool plan_windows(qm_ctx *ctx, const GroupTable &gt, int64_t n_rows, WindowPlan 
   if (windows > QM_WIN_MAX || ex.total_slots > ((int64_t)1 << QM_WIN_SLOT_BITS) ||
       qm_win_scatter_smem((int)windows, pl.agg.n_vcols) > QM_WIN_SMEM_MAX)
     return false;
+  {
+    qm_scan_args a;
+    fill_args(gt, a, (qm_status *)ctx->status.p);
+    if (qm_win_setup(a) != cudaSuccess) return false;
+  }
   const size_t rec_bytes = (size_t)n_rows * 8 * (1 + pl.agg.n_vcols);
   if (rec_bytes > (size_t)ctx->hbm_bytes / 8) return false;
   if (!wp.rec && !(wp.rec = col_alloc(ctx, rec_bytes, wp.rec_block))) return false;

@@ -154,6 +154,7 @@ cudaError_t qm_launch_part_agg(const qm_scan_args &a, const qm_part_spec &ps, in
 int qm_value_features(const qm_aggspec &A);  // QM_FT_*
 bool qm_win_supported(const qm_aggspec &A);
 size_t qm_win_scatter_smem(int windows, int n_vcols);
+cudaError_t qm_win_setup(const qm_scan_args &a);  // the plan's kernels can run on the current device
 cudaError_t qm_launch_windows(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st);
 
 // The library's exclusive scan: scratch bytes for n inputs, and ranks of a

@@ -23,6 +23,7 @@
 // so that the scatter's open write lines, one per (partition, block), stay
 // in L2 and reach DRAM as whole lines.
 #include "qm_kernels.cuh"
+#include "qm_device_once.h"
 #include "qm_launch.h"
 #include "qm_scan.cuh"
 
@@ -760,17 +761,20 @@ constexpr size_t PART_AGG_SMEM_MAX = 200 * 1024;
 
 template <auto Kernel>
 cudaError_t set_smem_once(size_t bytes, int *per_sm_out = nullptr) {
-  static std::once_flag once;  // one per kernel (the kernel is a template argument)
+  static qm_device_once once;  // one per kernel (the kernel is a template argument)
   const auto kernel = Kernel;
-  static cudaError_t err = cudaSuccess;
-  static int per_sm = 1;
-  std::call_once(once, [&] {
-    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (err == cudaSuccess)
-      err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, QM_SCAN_THREADS, bytes);
+  int device = 0;
+  cudaError_t err = cudaGetDevice(&device);
+  if (err != cudaSuccess) return err;
+  const qm_kernel_setup s = once.get(device, [&] {
+    int per_sm = 1;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, QM_SCAN_THREADS, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return qm_kernel_setup{(int)e, per_sm};
   });
-  if (per_sm_out) *per_sm_out = per_sm;
-  return err;
+  if (per_sm_out) *per_sm_out = s.per_sm;
+  return (cudaError_t)s.error;
 }
 
 template <int PASS, int NV, int KK>
@@ -867,39 +871,40 @@ cudaError_t qm_launch_part_agg(const qm_scan_args &a, const qm_part_spec &ps, in
 // ---- windows of a large direct table ----------------------------------------------
 
 namespace {
+// (ws null: only the kernels' shared memory limits are set)
 template <int KK>
-cudaError_t win_count(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
+cudaError_t win_count(const qm_scan_args &a, const qm_win_spec *ws, int sm_count, cudaStream_t st) {
   cudaError_t e = set_smem_once<qm_win_count<KK>>((size_t)QM_WIN_MAX * 4);
-  if (e != cudaSuccess) return e;
-  qm_win_count<KK><<<sm_count * 2, QM_SCAN_THREADS, (size_t)ws.windows * 4, st>>>(a, ws);
+  if (e != cudaSuccess || !ws) return e;
+  qm_win_count<KK><<<sm_count * 2, QM_SCAN_THREADS, (size_t)ws->windows * 4, st>>>(a, *ws);
   return cudaGetLastError();
 }
 
 template <int NV, int KK>
-cudaError_t win_scatter(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
+cudaError_t win_scatter(const qm_scan_args &a, const qm_win_spec *ws, int sm_count, cudaStream_t st) {
   cudaError_t e = set_smem_once<qm_win_scatter<NV, KK>>(QM_WIN_SMEM_MAX);
-  if (e != cudaSuccess) return e;
-  qm_win_scatter<NV, KK><<<sm_count, QM_WIN_THREADS, qm_win_scatter_smem(ws.windows, NV), st>>>(a, ws);
+  if (e != cudaSuccess || !ws) return e;
+  qm_win_scatter<NV, KK><<<sm_count, QM_WIN_THREADS, qm_win_scatter_smem(ws->windows, NV), st>>>(a, *ws);
   return cudaGetLastError();
 }
 
 template <int NV, int FT>
-cudaError_t win_agg(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
+cudaError_t win_agg(const qm_scan_args &a, const qm_win_spec *ws, int sm_count, cudaStream_t st) {
   cudaError_t e = set_smem_once<qm_win_agg<NV, FT>>(QM_WIN_SMEM_MAX);
-  if (e != cudaSuccess) return e;
-  qm_win_agg<NV, FT><<<sm_count, QM_WIN_THREADS, ((size_t)a.agg.n_words * 8) << ws.shift, st>>>(a, ws);
+  if (e != cudaSuccess || !ws) return e;
+  qm_win_agg<NV, FT><<<sm_count, QM_WIN_THREADS, ((size_t)a.agg.n_words * 8) << ws->shift, st>>>(a, *ws);
   return cudaGetLastError();
 }
 
 template <int NV>
-cudaError_t win_run(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
+cudaError_t win_run(const qm_scan_args &a, const qm_win_spec *ws, int sm_count, cudaStream_t st) {
   const int kk = part_key_kind(a.key);
   cudaError_t e = kk == QM_KK_I64   ? win_count<QM_KK_I64>(a, ws, sm_count, st)
                   : kk == QM_KK_I32 ? win_count<QM_KK_I32>(a, ws, sm_count, st)
                                     : win_count<QM_KK_ANY>(a, ws, sm_count, st);
   if (e != cudaSuccess) return e;
-  qm_win_offsets<<<1, QM_WIN_THREADS, 0, st>>>(ws);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (ws) qm_win_offsets<<<1, QM_WIN_THREADS, 0, st>>>(*ws);
+  if (ws && (e = cudaGetLastError()) != cudaSuccess) return e;
   e = kk == QM_KK_I64   ? win_scatter<NV, QM_KK_I64>(a, ws, sm_count, st)
       : kk == QM_KK_I32 ? win_scatter<NV, QM_KK_I32>(a, ws, sm_count, st)
                         : win_scatter<NV, QM_KK_ANY>(a, ws, sm_count, st);
@@ -921,11 +926,19 @@ size_t qm_win_scatter_smem(int windows, int n_vcols) {
   return (size_t)QM_WIN_ROWS * 8 * (1 + n_vcols) + (size_t)windows * 8;
 }
 
+cudaError_t qm_win_setup(const qm_scan_args &a) {
+  switch (a.agg.n_vcols) {
+    case 0: return win_run<0>(a, nullptr, 0, nullptr);
+    case 1: return win_run<1>(a, nullptr, 0, nullptr);
+    default: return win_run<2>(a, nullptr, 0, nullptr);
+  }
+}
+
 cudaError_t qm_launch_windows(const qm_scan_args &a, const qm_win_spec &ws, int sm_count, cudaStream_t st) {
   if (a.n <= 0) return cudaSuccess;
   switch (a.agg.n_vcols) {
-    case 0: return win_run<0>(a, ws, sm_count, st);
-    case 1: return win_run<1>(a, ws, sm_count, st);
-    default: return win_run<2>(a, ws, sm_count, st);
+    case 0: return win_run<0>(a, &ws, sm_count, st);
+    case 1: return win_run<1>(a, &ws, sm_count, st);
+    default: return win_run<2>(a, &ws, sm_count, st);
   }
 }
