@@ -163,8 +163,8 @@ struct PinnedPool {
   }
 };
 
-// Device blocks of destroyed tables' columns, kept (up to a cap) for the
-// next table's columns of about the same size: tables created and dropped
+// Device blocks of destroyed tables' columns and of large queries' scratch,
+// kept (up to a cap) for the next table's columns of about the same size: tables created and dropped
 // per host batch or per ingest then cost no cudaMalloc / cudaFree (and
 // cudaFree synchronises the device).  Emptied whenever an allocation fails.
 struct DevPool {
@@ -2483,20 +2483,25 @@ qm_pred with_key_range(const qm_pred &P, const qm_keyspec &K, int64_t lo, int64_
 // rows, 65,536 Zipf keys; uniform keys would take 2.2 -> 1.6).
 constexpr int64_t WINDOW_MIN_ROWS = 12000000;
 
-struct WindowPlan {  // device scratch of the call, back to the pool at its end
+// Device scratch of the windows, back in the context's pool as soon as their
+// launches are queued: what takes a pool block next orders its work behind
+// them on the context's stream, and an allocation of the same query that
+// fails empties the pool and has this memory.
+struct WindowPlan {
   qm_ctx *ctx;
   qm_win_spec spec{};
+  bool all_rows = false;  // records for every row: the sampled bound did not hold
   void *rec = nullptr, *meta = nullptr;
   size_t rec_block = 0, meta_block = 0;
   explicit WindowPlan(qm_ctx *c) : ctx(c) {}
   WindowPlan(const WindowPlan &) = delete;
   WindowPlan &operator=(const WindowPlan &) = delete;
-  ~WindowPlan() {
-    if (!rec && !meta) return;
-    cudaStreamSynchronize(ctx->stream);
+  void release() {
     col_release(ctx, rec, rec_block);
     col_release(ctx, meta, meta_block);
+    rec = meta = nullptr;
   }
+  ~WindowPlan() { release(); }
 };
 
 bool plan_windows(qm_ctx *ctx, const GroupTable &gt, int64_t n_rows, WindowPlan &wp) {
@@ -2519,15 +2524,16 @@ bool plan_windows(qm_ctx *ctx, const GroupTable &gt, int64_t n_rows, WindowPlan 
     fill_args(gt, a, (qm_status *)ctx->status.p);
     if (qm_win_setup(a) != cudaSuccess) return false;
   }
-  const size_t rec_bytes = (size_t)n_rows * 8 * (1 + pl.agg.n_vcols);
+  const int64_t cap = wp.all_rows ? n_rows : rows;
+  const size_t rec_bytes = (size_t)cap * 8 * (1 + pl.agg.n_vcols);
   if (rec_bytes > (size_t)ctx->hbm_bytes / 8) return false;
   if (!wp.rec && !(wp.rec = col_alloc(ctx, rec_bytes, wp.rec_block))) return false;
   if (!wp.meta && !(wp.meta = col_alloc(ctx, (size_t)(4 * QM_WIN_MAX + 16) * 4, wp.meta_block))) return false;
   ws.windows = (int)windows;
   ws.total_slots = ex.total_slots;
-  ws.rec_cap = n_rows;
+  ws.rec_cap = cap;
   // a window is one chunk unless it holds far more than its share of the rows
-  ws.chunk = std::max<int64_t>(n_rows / ((int64_t)ctx->sm_count * 8), 65536);
+  ws.chunk = std::max<int64_t>(cap / ((int64_t)ctx->sm_count * 8), 65536);
   ws.records = (uint64_t *)wp.rec;
   uint32_t *m = (uint32_t *)wp.meta;
   ws.counter = (int32_t *)m;  // cleared with the counts behind it
@@ -2538,7 +2544,7 @@ bool plan_windows(qm_ctx *ctx, const GroupTable &gt, int64_t n_rows, WindowPlan 
   return true;
 }
 
-int run_windows(qm_ctx *ctx, GroupTable &gt, int64_t n, const WindowPlan &wp) {
+int run_windows(qm_ctx *ctx, GroupTable &gt, int64_t n, WindowPlan &wp) {
   qm_scan_args a;
   fill_args(gt, a, (qm_status *)ctx->status.p);
   a.n = n;
@@ -2547,6 +2553,7 @@ int run_windows(qm_ctx *ctx, GroupTable &gt, int64_t n, const WindowPlan &wp) {
   CK(cudaMemsetAsync(wp.spec.counter, 0, (size_t)(4 + wp.spec.windows) * 4, ctx->stream));
   CK(qm_launch_windows(a, wp.spec, ctx->sm_count, ctx->stream));
   CK(cudaEventRecord(ctx->evs1, ctx->stream));
+  wp.release();
   ctx->launches += 4;
   gt.scan_pending = true;
   return QM_OK;
@@ -2999,6 +3006,7 @@ int qm_query_run(qm_ctx *ctx, const qm_table *table, const qm_query *q, qm_resul
   for (int attempt = 0;; attempt++) {
     gt.rows_done = 0;  // every attempt scans the table from its first row
     qm_status st;
+    bool windows = false;
     if ((rc = setup_table(ctx, gt, est, direct_size, false, false))) return rc;
     const bool tail = tail_query(ctx, gt, t->n_rows);
     if (tail) {
@@ -3026,7 +3034,7 @@ int qm_query_run(qm_ctx *ctx, const qm_table *table, const qm_query *q, qm_resul
       if (pp.on) {
         if ((rc = run_partitioned(ctx, gt, t->n_rows, pp))) return rc;
         gt.ex.strategy = 3;
-      } else if (plan_windows(ctx, gt, t->n_rows, wp)) {
+      } else if ((windows = plan_windows(ctx, gt, t->n_rows, wp))) {
         if ((rc = run_windows(ctx, gt, t->n_rows, wp))) return rc;
       } else if (passes <= 1) {
         if ((rc = run_scan(ctx, gt, t->n_rows, nullptr))) return rc;
@@ -3083,6 +3091,10 @@ int qm_query_run(qm_ctx *ctx, const qm_table *table, const qm_query *q, qm_resul
       for (int c = 0; c < pl.agg.n_vcols; c++)
         if (pl.vcolsrc[c]) const_cast<DevCol *>(pl.vcolsrc[c])->has_maxabs = false;
       if ((rc = plan_split_sums(ctx, pl, t->n_rows, true))) return rc;
+      continue;
+    }
+    if (windows && !wp.all_rows && st.error == QM_DEV_OVERFLOW) {
+      wp.all_rows = true;  // more rows selected than the sampled bound said
       continue;
     }
     if (st.error == QM_DEV_RANGE || pl.key.mode == QK_DIRECT) {
