@@ -31,6 +31,7 @@
 #include "../../include/qm_gpu.h"
 #include "qm_launch.h"
 #include "qm_plan.h"
+#include "qm_slots.h"
 
 typedef __int128 i128;
 
@@ -1061,20 +1062,6 @@ struct Exec {
 
 int64_t special_slots(int mode) { return mode == QK_HASH ? 2 : (mode == QK_DIRECT ? 1 : 0); }
 
-int ilog2_ceil(int64_t x) {
-  int l = 0;
-  while (((int64_t)1 << l) < x) l++;
-  return l;
-}
-
-// Slots of a hash table for an estimated number of groups: 2.1 each, any
-// number.  At 1.6 the longest of a warp's 32 probes grows (20M rows into
-// 500,000 groups: scan 0.76 -> 0.94 ms); rounded up to a power of two (2.1-4.3
-// each) the table is larger to clear, rank and emit and no faster to scan.
-int64_t hash_slots(int64_t groups) {
-  return std::min<int64_t>((int64_t)1 << 31, std::max<int64_t>(1024, groups * 2 + groups / 8));
-}
-
 constexpr size_t LOCAL_BUDGET = 40 * 1024;  // bytes of the block-local hash table
 constexpr size_t LOCAL_WIDE_BUDGET = 80 * 1024;  // ... when the estimated groups overflow it
 constexpr int64_t LOCAL_WIDE_MAX_GROUPS = 10000;
@@ -1714,7 +1701,7 @@ void fill_result(qm_result *R, const GroupTable &gt, const qm_outspec &O, int64_
   }
   R->stats.groups = G;
   R->stats.strategy = gt.ex.strategy;
-  R->stats.table_capacity = ilog2_ceil(std::max<int64_t>(gt.ex.n_slots, 1));
+  R->stats.table_capacity = qm_log2_ceil(std::max<int64_t>(gt.ex.n_slots, 1));
   R->stats.retries = gt.retries;
   R->stats.rows_selected = (int64_t)gt.selected;
   R->stats.scan_ms = gt.scan_ms;
@@ -2105,7 +2092,7 @@ int setup_table(qm_ctx *ctx, GroupTable &gt, int64_t est_groups, int64_t direct_
   } else {
     // a stream's table has room for the next batches' groups: a power of two,
     // as grow_table makes it
-    ex.n_slots = owned ? (int64_t)1 << std::min(31, ilog2_ceil(hash_slots(est_groups))) : hash_slots(est_groups);
+    ex.n_slots = owned ? (int64_t)1 << qm_log2_ceil(qm_hash_slots(est_groups)) : qm_hash_slots(est_groups);
   }
   choose_layout(pl, est_groups, ex, ctx->tuning, !owned);
   size_t bytes = (size_t)ex.total_slots * ex.stride * 8;
@@ -3188,11 +3175,10 @@ int stage_selection(qm_ctx *ctx, const uint32_t *sel, int64_t n_sel, const uint3
 // Grow a streaming hash table so that `upper` groups keep the load <= ~0.5.
 int grow_table(qm_ctx *ctx, GroupTable &gt, int64_t upper) {
   Exec &ex = gt.ex;
-  if (gt.pl.key.mode != QK_HASH || hash_slots(upper) <= ex.n_slots) return QM_OK;
+  const int log2cap = gt.pl.key.mode == QK_HASH ? qm_grown_log2(upper, ex.n_slots) : 0;
+  if (log2cap == 0) return QM_OK;
   Exec nx = ex;
-  // (a power of two: growing push by push re-hashes rarely)
-  const int log2cap = ilog2_ceil(hash_slots(upper));
-  if (log2cap > 31) return set_err(ctx, QM_ERR_OOM, "group table would exceed 2^31 slots");
+  if (log2cap > QM_MAX_LOG2_SLOTS) return set_err(ctx, QM_ERR_OOM, "group table would exceed 2^31 slots");
   nx.n_slots = (int64_t)1 << log2cap;
   nx.total_slots = nx.n_slots + 2;
   DevBuf nb;
@@ -3868,7 +3854,7 @@ extern "C" int qm_query_run_noalloc(qm_ctx *ctx, int64_t n_rows, int32_t n_cols,
   if (pl.key.mode == QK_NONE) {
     ex.n_slots = 1;
   } else {
-    const int log2cap = ilog2_ceil(std::max<int64_t>(1024, max_groups * 2 + max_groups / 8));
+    const int log2cap = qm_log2_ceil(std::max<int64_t>(1024, max_groups * 2 + max_groups / 8));
     if (log2cap > 30) return set_err(ctx, QM_ERR_CAPACITY, "max_groups too large for the scratch array");
     ex.n_slots = (int64_t)1 << log2cap;
   }
@@ -4662,7 +4648,7 @@ int batch_plan_one(qm_batch *b, int i, const qm_table *table, const qm_query *qu
   } else if (gt.pl.key.mode == QK_DIRECT) {
     ex.n_slots = direct_size;
   } else {
-    ex.n_slots = hash_slots(est);
+    ex.n_slots = qm_hash_slots(est);
   }
   choose_layout(gt.pl, est, ex, ctx->tuning, true);
   b->est[i] = est;
