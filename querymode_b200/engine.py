@@ -324,6 +324,26 @@ class _ResultOwner:
             pass
 
 
+# Page-locked bytes that the selections of a context hold at most, and a
+# selection's bytes up to which it is copied out: the library page-locks by
+# powers of two from 64 KB, and its memory cannot be swapped.
+SELECT_LENT_BYTES = 1 << 30
+SELECT_COPY_BYTES = 64 << 10
+
+
+class _LentOwner(_ResultOwner):
+    """A result counted in lent[0] while it lives."""
+
+    def __init__(self, lib, handle, lent: list, nbytes: int):
+        super().__init__(lib, handle)
+        self.lent, self.nbytes = lent, nbytes
+        lent[0] += nbytes
+
+    def __del__(self):
+        self.lent[0] -= self.nbytes
+        super().__del__()
+
+
 def _buffer_view(addr: int, nbytes: int, owner: _ResultOwner) -> np.ndarray:
     buf = (C.c_uint8 * max(nbytes, 1)).from_address(addr)
     buf._owner = owner  # the ctypes array keeps the result alive; numpy keeps the array
@@ -378,6 +398,7 @@ class Context:
         self.h = h
         self.device = device
         self._children = weakref.WeakSet()
+        self._lent = [0]  # page-locked bytes held by selections (filter_select)
 
     def _adopt(self, child) -> None:
         """Track a table / batch / stream / server made on this context: the
@@ -539,7 +560,11 @@ class Context:
     def filter_select(self, columns: Mapping[str, Any], query: QueryDescriptor,
                       selection: np.ndarray | None = None) -> np.ndarray:
         """Ascending indices of the rows (of `selection`, if given) passing
-        query's filters (a view of page-locked memory the array keeps)."""
+        query's filters.  A large selection is a view of page-locked memory
+        that the array keeps, up to SELECT_LENT_BYTES held by a context's
+        selections at a time; beyond that, where memory cannot be page-locked,
+        and below SELECT_COPY_BYTES (the least that is page-locked), it is an
+        array of its own."""
         cs = _ColumnSet(columns)
         cq = CQuery(query)
         sel_ptr, n_sel = None, 0
@@ -549,16 +574,26 @@ class Context:
             sel_ptr = sel.ctypes.data_as(C.POINTER(C.c_uint32))
             n_sel = sel.size
         r = C.c_void_p()
-        self.check(self.lib.qm_filter_select_result(self.h, cs.n_rows, cs.count, cs.array, cq.ref, sel_ptr, n_sel,
-                                                    C.byref(r)))
-        owner = _ResultOwner(self.lib, r)
+        status = self.lib.qm_filter_select_result(self.h, cs.n_rows, cs.count, cs.array, cq.ref, sel_ptr, n_sel, C.byref(r))
+        if status == A.QM_ERR_OOM:
+            cap = n_sel if selection is not None else cs.n_rows
+            out = np.empty(max(cap, 1), dtype=np.uint32)
+            cnt = C.c_int64()
+            self.check(self.lib.qm_filter_select(self.h, cs.n_rows, cs.count, cs.array, cq.ref, sel_ptr, n_sel,
+                                                 out.ctypes.data_as(C.POINTER(C.c_uint32)), cap, C.byref(cnt)))
+            return out[:cnt.value].copy()
+        self.check(status)
         n = C.c_int64()
         rc = A.QmResultCol()
         self.lib.qm_result_num_rows(r, C.byref(n))
         self.lib.qm_result_column(r, 0, C.byref(rc))
-        if n.value == 0:
+        nbytes = 4 * n.value
+        if nbytes > SELECT_COPY_BYTES and self._lent[0] + nbytes <= SELECT_LENT_BYTES:
+            return _buffer_view(rc.data, nbytes, _LentOwner(self.lib, r, self._lent, nbytes)).view(np.uint32)
+        owner = _ResultOwner(self.lib, r)
+        if nbytes == 0:
             return np.empty(0, dtype=np.uint32)
-        return _buffer_view(rc.data, 4 * n.value, owner).view(np.uint32)
+        return _buffer_view(rc.data, nbytes, owner).view(np.uint32).copy()
 
     def aggregate(self, query: QueryDescriptor) -> "AggStream":
         return AggStream(self, query)
