@@ -2092,7 +2092,8 @@ int setup_table(qm_ctx *ctx, GroupTable &gt, int64_t est_groups, int64_t direct_
   } else {
     // a stream's table has room for the next batches' groups: a power of two,
     // as grow_table makes it
-    ex.n_slots = owned ? (int64_t)1 << qm_log2_ceil(qm_hash_slots(est_groups)) : qm_hash_slots(est_groups);
+    ex.n_slots = owned ? (int64_t)1 << qm_log2_ceil(qm_hash_slots(est_groups))
+                       : qm_hash_slots(est_groups, ctx->tuning.dedupe > 0);
   }
   choose_layout(pl, est_groups, ex, ctx->tuning, !owned);
   size_t bytes = (size_t)ex.total_slots * ex.stride * 8;
@@ -4648,7 +4649,7 @@ int batch_plan_one(qm_batch *b, int i, const qm_table *table, const qm_query *qu
   } else if (gt.pl.key.mode == QK_DIRECT) {
     ex.n_slots = direct_size;
   } else {
-    ex.n_slots = qm_hash_slots(est);
+    ex.n_slots = qm_hash_slots(est, ctx->tuning.dedupe > 0);
   }
   choose_layout(gt.pl, est, ex, ctx->tuning, true);
   b->est[i] = est;

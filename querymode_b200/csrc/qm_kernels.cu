@@ -1642,6 +1642,7 @@ cudaError_t scan_attrs_once() {
   QM_SMEM_ATTR((qm_scan_kernel<false, true, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
   QM_SMEM_ATTR((qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
   QM_SMEM_ATTR((qm_scan_kernel<false, false, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
+  QM_SMEM_ATTR((qm_scan_kernel<false, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_HASH>));
   QM_SMEM_ATTR((qm_scan_kernel<true, false, 0, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
   QM_SMEM_ATTR((qm_scan_kernel<true, false, 1, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>));
 #undef QM_SMEM_ATTR
@@ -1702,8 +1703,8 @@ static scan_choice choose_scan(const qm_scan_args &a) {
 
 int qm_scan_kernel_id(const qm_scan_args &a) {
   const scan_choice c = choose_scan(a);
-  if (!c.spec) return (c.dd | (a.sel ? 2 : 0) | (a.stage.n > 0 ? 4 : 0));
-  return 8 + (((a.agg.n_vcols * 4 + c.kk) * 5 + c.ft) * 3 + c.lm) * 2 + c.dd;
+  if (!c.spec) return c.dd | (a.sel ? 2 : 0) | (a.stage.n > 0 ? 4 : 0) | (c.lm == QM_LM_HASH ? 8 : 0);
+  return 16 + (((a.agg.n_vcols * 4 + c.kk) * 5 + c.ft) * 3 + c.lm) * 2 + c.dd;
 }
 
 static cudaError_t scan_dispatch(const qm_scan_args &a, int blocks, size_t smem, cudaStream_t st, int *per_sm) {
@@ -1719,12 +1720,12 @@ static cudaError_t scan_dispatch(const qm_scan_args &a, int blocks, size_t smem,
       case 4: return qm_scan_nv4_launch(a, c.dd, c.kk, c.ft, c.lm, blocks, smem, st, per_sm);
     }
   }
-#define QM_GENERIC(SEL, STAGED, DD)                                                                                \
-  launch_scan_kernel(qm_scan_kernel<SEL, STAGED, DD, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, QM_LM_ANY>, a, blocks, smem, \
-                     st, per_sm)
-  if (a.sel) return c.dd ? QM_GENERIC(true, false, 1) : QM_GENERIC(true, false, 0);
-  if (a.stage.n > 0) return c.dd ? QM_GENERIC(false, true, 1) : QM_GENERIC(false, true, 0);
-  return c.dd ? QM_GENERIC(false, false, 1) : QM_GENERIC(false, false, 0);
+#define QM_GENERIC(SEL, STAGED, DD, LM)                                                                                  \
+  launch_scan_kernel(qm_scan_kernel<SEL, STAGED, DD, QM_NV_ANY, QM_KK_ANY, QM_FT_FULL, LM>, a, blocks, smem, st, per_sm)
+  if (a.sel) return c.dd ? QM_GENERIC(true, false, 1, QM_LM_ANY) : QM_GENERIC(true, false, 0, QM_LM_ANY);
+  if (a.stage.n > 0) return c.dd ? QM_GENERIC(false, true, 1, QM_LM_ANY) : QM_GENERIC(false, true, 0, QM_LM_ANY);
+  if (c.dd) return QM_GENERIC(false, false, 1, QM_LM_ANY);
+  return c.lm == QM_LM_HASH ? QM_GENERIC(false, false, 0, QM_LM_HASH) : QM_GENERIC(false, false, 0, QM_LM_ANY);
 #undef QM_GENERIC
 }
 

@@ -12,16 +12,19 @@ constexpr int QM_MAX_LOG2_SLOTS = 31;
 // to clear, rank and emit.
 inline int64_t qm_slots_wanted(int64_t groups) { return std::max<int64_t>(1024, groups * 2 + groups / 8); }
 
-// Slots of a one-shot table (a table too small for its groups overflows and
-// is made again).
-inline int64_t qm_hash_slots(int64_t groups) {
-  return std::min<int64_t>((int64_t)1 << QM_MAX_LOG2_SLOTS, qm_slots_wanted(groups));
-}
-
 inline int qm_log2_ceil(int64_t x) {
   int l = 0;
   while (((int64_t)1 << l) < x) l++;
   return l;
+}
+
+// Slots of a one-shot table (a table too small for its groups overflows and
+// is made again).  Deduplicating kernels read the key alone while they probe,
+// so for them it is rounded up to a power of two (20M rows into 2,000 groups,
+// five columns: scan 2.39 -> 1.90 ms).
+inline int64_t qm_hash_slots(int64_t groups, bool dedupe = false) {
+  const int64_t want = std::min<int64_t>((int64_t)1 << QM_MAX_LOG2_SLOTS, qm_slots_wanted(groups));
+  return dedupe ? (int64_t)1 << qm_log2_ceil(want) : want;
 }
 
 // log2 of the slots a stream's table of n_slots grows to for `groups` groups:
