@@ -62,6 +62,18 @@ __host__ __device__ inline smem_layout make_smem_layout(int local_slots, int loc
 // NV / KK: the value-column count and key kind the kernel is specialised
 // for (QM_NV_ANY / QM_KK_ANY: read from the plan at run time); FT / LM: what
 // its value columns need and where its rows go (QM_FT_*, QM_LM_*).
+// The first of a lane's n places in the queue, and the warp's total.
+__device__ __forceinline__ uint32_t warp_places(uint32_t n, int lane, uint32_t &total) {
+  uint32_t off = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(QM_FULL, off, o);
+    if (lane >= o) off += x;
+  }
+  total = __shfl_sync(QM_FULL, off, 31);
+  return off - n;
+}
+
 template <bool SEL, bool STAGED, int DD, int NV, int KK, int FT, int LM>
 __global__ void __launch_bounds__(QM_SCAN_THREADS)
     qm_scan_kernel(const __grid_constant__ qm_scan_args a) {
@@ -175,7 +187,8 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
     const int tile = tile_of(v);
     if (tile >= n_tiles) continue;  // the table's last zone is partial
     const int64_t e0 = (int64_t)tile * tile_rows;
-    uint32_t m = 0, left = 0;  // left: rows of m, of all lanes, that are not in the queue yet
+    uint32_t m = 0;
+    bool fill = false;  // m's rows are not in the queue yet
     if (STAGED && tile < full_tiles) {
       __syncwarp();
       issue(k + S.depth - 1);
@@ -236,22 +249,18 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
           m |= eval_pred(a.pred, rowf, mh) << (h * QM_R);
         }
       }
-      left = __reduce_add_sync(QM_FULL, __popc(m));
-      selected += left;
+      fill = true;
     }
     do {
-      if (left) {  // (order inside the queue does not matter: FIRST is a min)
-        const uint32_t now = qn + left <= QM_WQ ? m : m & ((1u << QM_R) - 1);
-        m ^= now;
-        const uint32_t cnt = __popc(now);
-        uint32_t off = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t x = __shfl_up_sync(QM_FULL, off, o);
-          if (lane >= o) off += x;
+      if (fill) {  // (order inside the queue does not matter: FIRST is a min)
+        uint32_t now = m, tot;
+        uint32_t q = qn + warp_places(__popc(now), lane, tot);
+        fill = qn + tot > QM_WQ;
+        if (fill) {  // the first tile's rows, then the second's
+          now &= (1u << QM_R) - 1;
+          m ^= now;
+          q = qn + warp_places(__popc(now), lane, tot);
         }
-        const uint32_t tot = __shfl_sync(QM_FULL, off, 31);
-        uint32_t q = qn + off - cnt;
         const uint32_t r0u = (uint32_t)(e0 + lane * QM_R);
         for (uint32_t mm = now; mm; mm &= mm - 1) {
           const uint32_t j = (uint32_t)(__ffs(mm) - 1);
@@ -259,14 +268,14 @@ __global__ void __launch_bounds__(QM_SCAN_THREADS)
           queue[q++] = SEL ? __ldg(a.sel + row) : row;
         }
         qn += (int)tot;
-        left -= tot;
+        selected += tot;
       }
       __syncwarp();
       while (qn >= 32 * D) {
         drain(qn - 32 * D, 32 * D);
         qn -= 32 * D;
       }
-    } while (left);
+    } while (fill);
   }
   if (STAGED && failed) {
     // let every copy still in flight land before the block's memory goes
