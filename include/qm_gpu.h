@@ -247,10 +247,13 @@ const char *qm_ctx_last_error(const qm_ctx *ctx);
 int qm_ctx_set_stream(qm_ctx *ctx, void *stream);
 /* Set (tuning != NULL) or clear (NULL) the context's launch-shape knobs. */
 int qm_ctx_set_tuning(qm_ctx *ctx, const qm_tuning *tuning);
-/* Device blocks of destroyed tables are kept by the context for the next
- * tables of about their size (up to an eighth of the device's memory; given
- * back by this library whenever one of its allocations fails, and at
- * qm_ctx_destroy).  Batch and serving buffers come from the device's
+/* Device blocks of destroyed tables, and the records of a large roll-up
+ * (qm_query_run over a dense key range of more than a million groups: 8 bytes
+ * a selected row and 8 more for each of up to two value columns, 3.2 GB for
+ * 200M rows and one column, never more than an eighth of the device's memory),
+ * are kept by the context for the next ones of about their size (up to an
+ * eighth of the device's memory; given back by this library whenever one of
+ * its allocations fails, and at qm_ctx_destroy).  Batch and serving buffers come from the device's
  * stream-ordered memory pool and stay in it when freed.  This frees both
  * now, for a caller whose other allocators need the memory; *released (may
  * be null) receives the table-block bytes freed.  No counterpart in the
@@ -593,8 +596,9 @@ typedef struct {
 /* Start the lanes.  At creation the server page-locks 256 MB of result
  * buffers per lane (kept in the context's pinned pool) and takes up to 2 GB
  * per lane (at most an eighth of hbm_budget_bytes) from the device's memory
- * pool and hands it back, so that serving does not stall on page-locking or
- * pool growth later; qm_ctx_trim returns the device memory. */
+ * pool and hands it back, except half of it, which the lanes keep for their
+ * group tables until qm_server_destroy, so that serving does not stall on
+ * page-locking or pool growth later; qm_ctx_trim returns the rest. */
 int qm_server_create(qm_ctx *ctx, const qm_server_config *cfg, qm_server **out);
 /* Queue one request (the query is copied; the table must stay alive).
  * *ticket identifies it for cancel / wait.  Planning errors surface from

@@ -1117,9 +1117,10 @@ void choose_layout(const Plan &pl, int64_t est_groups, Exec &ex, const qm_tuning
   if (tu.local_slots > 0 || (tu.local_slots == 0 && est_groups <= ((int64_t)1 << 20))) {
     int L = 1;
     while ((int64_t)(L * 2) * (per_slot + 8) <= (int64_t)LOCAL_BUDGET) L *= 2;
-    // More groups than that table admits (half its slots): a wider table,
-    // still two blocks per SM, keeps them in shared memory (256-1,000
-    // int64 groups at 75 % selectivity: 3.9 -> 1.9 ms over 15 queries).
+    // Beyond half of that table's slots its buckets of four fill up: a wider
+    // table, still two blocks per SM, keeps the groups in shared memory
+    // (256-1,000 int64 groups at 75 % selectivity: 3.9 -> 1.9 ms over 15
+    // queries).
     if (tu.local_slots == 0 && est_groups > L / 2 && est_groups <= LOCAL_WIDE_MAX_GROUPS)
       while ((int64_t)(L * 2) * (per_slot + 8) <= (int64_t)LOCAL_WIDE_BUDGET) L *= 2;
     if (tu.local_slots > 0) {

@@ -55,8 +55,8 @@ __global__ void qm_batch_init(const qm_bq *bq, const int64_t *slot0, int n, int6
   }
 }
 
-// Shared memory: block-local table (keys, then words SoA), per-warp queues,
-// per-warp merge scratch — sized for the batch's largest local table.
+// Shared memory: block-local table (keys, then words SoA) and per-warp queues,
+// sized for the batch's largest local table.
 struct bsmem {
   size_t words_off, queue_off, bytes;
 };

@@ -164,8 +164,6 @@ __global__ void qm_init_table(uint64_t *t, int64_t n_slots_total, int stride, in
   }
 }
 
-// Occupied slots (COUNT word > 0) with their sort key: the first-seen row
-// (or the slot itself when no order is needed).
 __device__ __forceinline__ uint64_t global_timer() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -282,6 +280,8 @@ __global__ void __launch_bounds__(256) qm_tail_init(uint64_t *t, int n_words_tot
   }
 }
 
+// Occupied slots (COUNT word > 0) with their sort key: the first-seen row
+// (or the slot itself when no order is needed).
 __global__ void qm_compact_groups(const uint64_t *t, int64_t n_slots_total, int stride, int count_word,
                                   int first_word, uint64_t *keys_out, uint32_t *slots_out,
                                   unsigned long long *counter) {
