@@ -763,6 +763,11 @@ __global__ void __launch_bounds__(QM_STAT_THREADS) qm_col_stats(const T *p, cons
   constexpr bool FLT = (T)0.5 != (T)0;
   const int64_t r0 = (int64_t)blockIdx.x * QM_STAT_ROWS;
   stat_acc s;
+  // the sampled cells, read ahead of the chunk
+  constexpr int STEP = QM_STAT_ROWS / QM_STAT_SAMPLES;
+  const int64_t sampled = r0 + threadIdx.x * STEP + (blockIdx.x * 0x9e3779b1u >> 16) % STEP;
+  T cell = 0;
+  if (FLT && threadIdx.x < QM_STAT_SAMPLES && sampled < n && !cell_null(nulls, sampled)) cell = p[sampled];
   if (aligned && r0 + QM_STAT_ROWS <= n) {
     for (int i = 0; i < ITERS; i += 8) {
       V x[8];
@@ -810,20 +815,15 @@ __global__ void __launch_bounds__(QM_STAT_THREADS) qm_col_stats(const T *p, cons
     qm_chunk_stat &r = out[blockIdx.x];
     r.mn = FLT ? __double_as_longlong(ord2f(s.mn)) : s.mn;
     r.mx = FLT ? __double_as_longlong(ord2f(s.mx)) : s.mx;
-    r.count = s.cnt;
+    r.count = (int32_t)s.cnt;
     r.maxabs = ab;
   }
   if (threadIdx.x < QM_STAT_SAMPLES) {
-    constexpr int STEP = QM_STAT_ROWS / QM_STAT_SAMPLES;
-    const int64_t row = r0 + threadIdx.x * STEP + (blockIdx.x * 0x9e3779b1u >> 16) % STEP;
+    const long long b = __double_as_longlong((double)cell);
+    const int ex = (int)((b >> 52) & 0x7ff);
+    const long long m = (b & ((1LL << 52) - 1)) | (ex ? 1LL << 52 : 0);
     int16_t low = QM_NO_BIT;
-    if (FLT && row < n && !cell_null(nulls, row)) {
-      const double d = (double)p[row];
-      const long long b = __double_as_longlong(d);
-      const int ex = (int)((b >> 52) & 0x7ff);
-      const long long m = (b & ((1LL << 52) - 1)) | (ex ? 1LL << 52 : 0);
-      if (ex != 0x7ff && m != 0) low = (int16_t)((ex ? ex : 1) - 1075 + __ffsll(m) - 1);
-    }
+    if (FLT && ex != 0x7ff && m != 0) low = (int16_t)((ex ? ex : 1) - 1075 + __ffsll(m) - 1);
     out[blockIdx.x].low[threadIdx.x] = low;
   }
 }

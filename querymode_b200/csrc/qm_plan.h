@@ -27,15 +27,15 @@
 // Column statistics are taken in chunks of this many rows (a divisor of a zone).
 #define QM_STAT_ROWS 8192
 #define QM_STAT_THREADS 256
-#define QM_STAT_SAMPLES 4
+#define QM_STAT_SAMPLES 2
 #define QM_NO_BIT 0x7fff
 struct qm_chunk_stat {
   int64_t mn, mx;   // integer columns: values; float columns: double bits
-  int64_t count;    // non-NULL cells (floats: that are not NaN)
   int64_t maxabs;   // float columns: bits of the largest finite |x|
   // float columns: the exponent of the lowest set bit of QM_STAT_SAMPLES of the
   // chunk's cells (QM_NO_BIT: NULL, zero, not finite, or past the end)
   int16_t low[QM_STAT_SAMPLES];
+  int32_t count;    // non-NULL cells (floats: that are not NaN)
 };
 // Rows a warp of the scan takes at a time where every warp has enough: two
 // tiles, so that the plan's term fields, the compaction and the loop are paid
