@@ -14,6 +14,10 @@ result's copy back to the host.
            from pinned memory, query, result download, every step
   roofline the fused scan kernel: algorithmic bytes per launch / its average
            CUDA-event duration, against the measured HBM copy bandwidth
+           (algorithmic: every referenced column in full, although columns
+           behind a selective filter are read only where rows remain, so a
+           frac above 1 is no error; traffic_frac takes the DRAM bytes of the
+           committed profile instead)
   cpu_baseline  the CPU oracle (a C restatement of the reference's JS path)
            on a bounded sample, rank 0, N=1 only
 
@@ -295,7 +299,8 @@ def run_config(ctx, stream, name: str, cols: dict, q, bytes_per_row: int, steps:
         "rows_selected": int(res.stats.rows_selected), "steps": steps, "warmup": max(3, warmup),
         "ms_per_query": ms, "value": qbytes / (ms / 1e3) / 1e9, "unit": "GB/s", "rows_per_s": n / (ms / 1e3),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "peak_kind": peak_kind, "kernel": "qm_scan_kernel", "kernel_ms": scan_ms},
+                     "bytes": "all referenced columns, read or not", "peak_kind": peak_kind,
+                     "kernel": "qm_win_*" if name.endswith("unfiltered") else "qm_scan_kernel", "kernel_ms": scan_ms},
         "e2e": e2e, "cpu_baseline": cpu,
         "parity": None if parity is None else parity["ok"], "parity_check": parity, "gpu_launches": launches,
         "note": note,
@@ -897,7 +902,9 @@ def main():
                        "l2": f"inputs {n * BYTES_PER_ROW / 1e9:.2f} GB per GPU > 126 MB L2 (no flush needed)",
                        "parallelism": f"dp{world}" + (" (row shards, partial states gathered to rank 0 over NCCL, merged there)" if world > 1 else "")},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
+                         "frac": achieved / peak, "traffic": traffic,
+                         "traffic_frac": traffic / (scan_avg / 1e3) / 1e9 / peak if traffic else None,
+                         "bytes": "all referenced columns, read or not", "peak_kind": peak_kind,
                          "kernel": "qm_scan_kernel", "kernel_ms": scan_avg},
             "parity": None if parity is None else parity["ok"],
             "parity_check": parity,

@@ -986,6 +986,7 @@ __device__ __forceinline__ void apply_row(const qm_aggspec &A, uint64_t *tp, int
   auto iadd = [](int64_t x, int64_t y) { return x + y; };
   auto fadd = [](double x, double y) { return x + y; };
   for (int i = 0; i < A.n_accs; ++i) {
+    __syncwarp(act);  // the lanes part ways at their probes and at each update: meet again
     const qm_acc ac = A.acc[i];
     uint64_t *w0 = tp ? tp + (int64_t)ac.word * ws : nullptr;
     uint64_t *w1 = tp ? tp + (int64_t)(ac.word + 1) * ws : nullptr;
